@@ -32,7 +32,8 @@ __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(_
 // (x, y) as packed bf16: the rounded values, and what the rounding left over
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16(x, y);
-  lo = pack_bf16(x - bf16_lo(hi), y - bf16_hi(hi));
+  const float2 rest = fma_f32x2(make_float2(bf16_lo(hi), bf16_hi(hi)), make_float2(-1.f, -1.f), make_float2(x, y));      // (exact)
+  lo = pack_bf16(rest.x, rest.y);
 }
 
 // d += a * b with a, b given as high and low parts

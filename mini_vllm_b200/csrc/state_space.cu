@@ -6,7 +6,8 @@
 // Everything behind the projections and the short convolution (whose outputs x, B and C come in the activation type) is fp32: dt, the
 // decays and their logarithms, the state.  State slots: [slots, heads, N, vp] fp32, vp = vdim rounded up to 4.
 //
-// Ragged step, bf16 (ssd_chunk_kernel): chunks of 64 tokens.  With F_t = sum_{s <= t} a dt_s inside a chunk and its initial S0:
+// Ragged step, bf16: decay_chunk_kernel (decay_chunks.cuh) where sizes, alignment and prompt lengths allow it, else
+// ssd_chunk_kernel: chunks of 64 tokens.  With F_t = sum_{s <= t} a dt_s inside a chunk and its initial S0:
 //   y_t = e^{F_t} S0^T C_t + sum_{s <= t} M_ts x_s          M_ts = (C_t . B_s) e^{F_t - F_s} dt_s,  + D where t = s
 //   S  <- e^{F_64} S0 + sum_s B_s (e^{F_64 - F_s} dt_s x_s)^T
 // All exponents are <= 0, so no factor exceeds 1 whatever the steps are.  A CTA walks the chunks of one sequence for one head and 16
@@ -26,8 +27,11 @@
 //
 // Roofline: HBM for all of them (decode: 8 N vdim bytes per head and sequence); the chunk kernel is held by mma.sync issue.
 #include "chunk_common.cuh"
+#include "decay_chunks.cuh"
 #include "host_util.cuh"
 #include "mini_vllm_b200.h"
+
+#include <algorithm>
 
 namespace mvb {
 
@@ -548,6 +552,15 @@ static int ssd_segment(int tokens, int longest, int heads, int vdim) {
 }
 static int64_t ssd_segment_slots(int tokens, int num_seqs, int seg) { return tokens / seg + num_seqs; }
 
+// The same for decay_chunk_kernel, which has an SM to itself
+static int ssd_wide_segment(int tokens, int longest, int heads, int vdim) {
+  const int64_t work = static_cast<int64_t>(tokens) * heads * (vdim / 64), room = sm_count();
+  if (longest < 1024 || longest > tokens || longest * room <= 2 * work) return 0;
+  int seg = 256;
+  while (seg < 1024 && work / (2 * seg) >= 2 * room) seg *= 2;
+  return seg;
+}
+
 template <int KS, int WARPS, bool STATES>
 static int launch_ssd_pass(const SsdParams& p, cudaStream_t st) {
   using G = SsdCfg<KS, WARPS, STATES>;
@@ -571,6 +584,29 @@ static int launch_ssd_chunks(const SsdParams& p, cudaStream_t st) {
   return launch_ssd_pass<KS, WARPS, false>(p, st);
 }
 
+// decay_chunk_kernel over whole sequences or segments
+template <int KB>
+static int launch_ssd_wide(const SsdParams& p, cudaStream_t st) {
+  CUtensorMap maps[3];
+  int rc = decay_maps(maps, p.c, p.b, p.x, p.stride, p.tokens, p.heads / p.per_group, p.n, p.heads, p.vdim);
+  if (rc != kOk) return rc;
+  DecayChunkParams d{};
+  d.a = static_cast<const __nv_bfloat16*>(p.dt); d.a_stride = p.dt_stride; d.a_bias = p.dt_bias; d.a_log2e = p.a_log2e; d.skip = p.d;
+  d.q_scale = 1.f; d.cap = 1.f;
+  d.y = static_cast<__nv_bfloat16*>(p.y); d.y_stride = p.y_stride;
+  d.state = p.state; d.slots = p.slots; d.num_slots = p.num_slots; d.cu = p.cu; d.positions = p.positions;
+  d.num_seqs = p.num_seqs; d.heads = p.heads; d.per_group = p.per_group; d.n = p.n; d.vdim = p.vdim; d.vp = p.vp;
+  d.seg = p.seg; d.seg_state = p.seg_state; d.seg_keep = p.seg_keep; d.dev_status = p.dev_status;
+  const unsigned z = p.seg == 0 ? p.num_seqs : static_cast<unsigned>(ssd_segment_slots(p.tokens, p.num_seqs, p.seg));
+  if (p.seg != 0) {
+    rc = launch_decay_pass<KB, false, true>(maps, d, z, st);
+    if (rc != kOk) return rc;
+    ssd_join_kernel<<<dim3((p.n * p.vp / 4 + 255) / 256, p.heads, p.num_seqs), 256, 0, st>>>(p);
+    if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+  }
+  return launch_decay_pass<KB, false, false>(maps, d, z, st);
+}
+
 template <int KS>
 static int launch_ssd_columns(const SsdParams& p, cudaStream_t st) {
   const int tiles = (p.vdim + 15) / 16;
@@ -587,10 +623,11 @@ static int launch_ssd_tokens(const SsdParams& p, cudaStream_t st) {
 }
 
 template <class T>
-static int launch_ssd(const SsdParams& p, cudaStream_t st) {
+static int launch_ssd(const SsdParams& p, bool wide, cudaStream_t st) {
   if (p.cu == nullptr) return launch_ssd_step<T>(p, st);
   if (p.heads > 65535 || p.num_seqs > 65535 || (p.seg != 0 && ssd_segment_slots(p.tokens, p.num_seqs, p.seg) > 65535)) return kUnsupportedShape;
   if constexpr (sizeof(T) == 2) {
+    if (wide) return p.n == 64 ? launch_ssd_wide<1>(p, st) : launch_ssd_wide<2>(p, st);
     switch (chunk_ks(p.n)) {
       case 1: return launch_ssd_columns<1>(p, st);
       case 2: return launch_ssd_columns<2>(p, st);
@@ -710,9 +747,11 @@ extern "C" size_t mvb_state_space_scratch_bytes(int dtype, int num_tokens, int n
                                                 int ragged) {
   using namespace mvb;
   if (!ragged || dtype != kBf16 || num_seqs <= 0 || heads <= 0 || num_states <= 0 || vdim <= 0) return 0;
-  const int seg = ssd_segment(num_tokens, longest, heads, vdim);
-  if (seg == 0) return 0;
-  return static_cast<size_t>(ssd_segment_slots(num_tokens, num_seqs, seg)) * heads * (static_cast<size_t>(num_states) * ((vdim + 3) / 4 * 4) + 1) * sizeof(float);
+  // alignment, which decides between the kernels, is not known here: enough for either
+  int64_t slots = 0;
+  for (int seg : {ssd_segment(num_tokens, longest, heads, vdim), ssd_wide_segment(num_tokens, longest, heads, vdim)})
+    if (seg != 0) slots = std::max(slots, ssd_segment_slots(num_tokens, num_seqs, seg));
+  return static_cast<size_t>(slots) * heads * (static_cast<size_t>(num_states) * ((vdim + 3) / 4 * 4) + 1) * sizeof(float);
 }
 
 extern "C" int mvb_state_space(int dtype, const void* x, const void* b, const void* c, int64_t xbc_row_stride, const void* dt,
@@ -734,7 +773,9 @@ extern "C" int mvb_state_space(int dtype, const void* x, const void* b, const vo
   SsdParams p{x, b, c, xbc_row_stride, dt, dt_row_stride, dt_bias, a_log2e, d, y, y_row_stride, state, state_slots, num_slots,
                     cu_seqlens_q, positions, num_seqs, num_tokens, heads, heads / groups, num_states, vdim, (vdim + 3) / 4 * 4, vec, 0, nullptr,
               nullptr, dev_status};
-  if (dtype == kBf16 && cu_seqlens_q != nullptr) p.seg = ssd_segment(num_tokens, longest, heads, vdim);
+  const bool wide = dtype == kBf16 && cu_seqlens_q != nullptr && vec && decay_chunks_fit(c, b, x, xbc_row_stride, num_states, vdim, num_tokens, num_seqs, heads);
+  if (dtype == kBf16 && cu_seqlens_q != nullptr)
+    p.seg = wide ? ssd_wide_segment(num_tokens, longest, heads, vdim) : ssd_segment(num_tokens, longest, heads, vdim);
   if (p.seg != 0) {
     if (!scratch || scratch_bytes < mvb_state_space_scratch_bytes(dtype, num_tokens, num_seqs, longest, heads, num_states, vdim, 1)) return kInvalidArgument;
     if (!is_aligned(scratch, 16)) return kMisaligned;
@@ -742,7 +783,7 @@ extern "C" int mvb_state_space(int dtype, const void* x, const void* b, const vo
     p.seg_keep = p.seg_state + ssd_segment_slots(num_tokens, num_seqs, p.seg) * heads * num_states * p.vp;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return dtype == kBf16 ? launch_ssd<__nv_bfloat16>(p, st) : launch_ssd<float>(p, st);
+  return dtype == kBf16 ? launch_ssd<__nv_bfloat16>(p, wide, st) : launch_ssd<float>(p, false, st);
 }
 
 extern "C" int mvb_gated_group_norm(int dtype, const void* y, int64_t y_row_stride, const void* z, int64_t z_row_stride, const float* weight,

@@ -1,0 +1,93 @@
+"""decay_chunk_kernel (recurrences with one decay per head, 128 tokens at a time) at the edges of its chunks, operand blocks and segments,
+through the entry points that reach it, against the plain oracles.  Tolerances are those of the same entry points elsewhere: outputs are
+rounded to bf16 (2^-9 of a value) and every factor has 16 bits."""
+import math
+
+import pytest
+import torch
+
+from mini_vllm_b200 import _cabi, ops
+from oracle import vebonex as memory
+from tests.step_helpers import gen, rel, run_steps
+from tests.test_gpu_rasezen_ops import run_state_space, want_state_space
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def space_inputs(g, lens, heads, groups, n, vdim):
+    mk = lambda *s: torch.randn(*s, generator=g).to(BF)
+    return [{"x": mk(t, heads, vdim), "b": mk(t, groups, n), "c": mk(t, groups, n), "dt": mk(t, heads)} for t in lens]
+
+
+@pytest.mark.parametrize("n,vdim", [(64, 64), (128, 64), (128, 128)])
+@pytest.mark.parametrize("dt_bias,log_a", [(-4.0, 1.5), (-30.0, 0.0), (40.0, 3.0), (-1.0, -12.0)])
+def test_state_space_edges(cuda, n, vdim, dt_bias, log_a):
+    g, heads = gen(n + vdim), 4
+    seqs = space_inputs(g, [1, 31, 127, 128, 129, 256, 300, 400], heads, 2, n, vdim)
+    bias, a, d = torch.full((heads,), dt_bias), -torch.exp(log_a + torch.randn(heads, generator=g) * 0.1), torch.randn(heads, generator=g)
+    for portions in ([[10 ** 6]], [[128, 33], [65, 1, 200]]):
+        for x, s in zip(run_state_space(cuda, seqs, heads, bias, a, d, portions, BF), seqs):
+            assert rel(x, want_state_space(s, bias, a, d)) < 6e-3
+
+
+@pytest.mark.parametrize("n,vdim", [(64, 128), (128, 64)])
+def test_state_space_segments(cuda, n, vdim):
+    g, heads, lens = gen(n), 2, [1500, 71, 1, 1280]
+    assert _cabi.load().mvb_state_space_scratch_bytes(0, sum(lens), len(lens), max(lens), heads, n, vdim, 1) > 0
+    seqs = space_inputs(g, lens, heads, 1, n, vdim)
+    bias, a, d = torch.full((heads,), -3.0), -torch.exp(torch.linspace(-9, 1, heads)), torch.ones(heads)
+    for portions in ([[10 ** 6]], [[1100, 64, 300], [70, 1], [1], [1200]]):
+        for x, s in zip(run_state_space(cuda, seqs, heads, bias, a, d, portions, BF), seqs):
+            assert rel(x, want_state_space(s, bias, a, d)) < 6e-3
+
+
+def test_a_neighbour_full_of_infinities(cuda):
+    """What lies behind a sequence's last row in memory is read, and must not reach its outputs or its state."""
+    g, heads = gen(1), 2
+    seqs = space_inputs(g, [130, 70, 200, 5], heads, 1, 128, 64)
+    for bad in (seqs[1], seqs[3]):
+        for k in ("x", "b", "c"):
+            bad[k][:] = math.inf
+    bias, a, d = torch.zeros(heads), torch.tensor([-0.3, -2.0]), torch.ones(heads)
+    got = run_state_space(cuda, seqs, heads, bias, a, d, [[10 ** 6], [10 ** 6], [77], [10 ** 6]], BF)
+    for i in (0, 2):
+        assert rel(got[i], want_state_space(seqs[i], bias, a, d)) < 6e-3
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128), (128, 64), (64, 192)])
+@pytest.mark.parametrize("f_bias,swing", [(4.0, 1.0), (-8.0, 6.0), (0.0, 20.0)])
+def test_matrix_memory_edges(cuda, dim, vdim, f_bias, swing):
+    g, heads, cap, lens = gen(dim + vdim), 3, 15.0, [1, 31, 127, 128, 129, 300]
+    mk = lambda *s: torch.randn(*s, generator=g).to(BF)
+    seqs = [{"q": mk(t, heads, dim), "k": mk(t, heads, dim), "v": mk(t, heads, vdim), "gate": mk(t, heads * vdim),
+             "f": (mk(t, heads) * swing).to(BF), "i": (mk(t, heads) * swing).to(BF)} for t in lens]
+    fb, ib, nw = torch.full((heads,), f_bias), torch.full((heads,), -2.0), torch.rand(heads * vdim, generator=g) + 0.5
+    capped = lambda x, bias: cap * torch.tanh((x.double() + bias.double()) / cap)
+    want = []
+    for s in seqs:
+        x = {k: v.double() for k, v in s.items()}
+        f, i = torch.nn.functional.logsigmoid(capped(s["f"], fb)), capped(s["i"], ib)
+        o = torch.stack([memory.mlstm_memory(x["q"][:, h] * dim ** -0.5, x["k"][:, h], x["v"][:, h], i[:, h], f[:, h])[0] for h in range(heads)], dim=1)
+        o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-6)
+        want.append(o.flatten(1) * nw.double() * torch.sigmoid(x["gate"]))
+    for portions in ([[10 ** 6]], [[128, 33], [65, 1, 200]]):
+        n = len(seqs)
+        states = tuple(torch.full(s, 3.0, device=cuda) for s in ((n + 2, heads, dim, vdim), (n + 2, heads, dim), (n + 2, heads)))
+        got, status = [torch.full(w.shape, math.nan, dtype=torch.float64) for w in want], ops.new_status(cuda)
+
+        def step(entries, cu, pos, slot):
+            x = {k: torch.cat([seqs[i][k][lo:hi] for i, lo, hi in entries]).to(cuda) for k in seqs[0]}
+            wide = torch.cat([x[k].flatten(1) for k in ("q", "k", "v")], dim=1)
+            q, k, v = wide.split([heads * dim, heads * dim, heads * vdim], dim=1)
+            out = torch.full((pos.numel(), heads, vdim), math.nan, dtype=BF, device=cuda)
+            ops.mlstm(q.unflatten(1, (heads, dim)), k.unflatten(1, (heads, dim)), v.unflatten(1, (heads, vdim)), x["f"], fb.to(cuda), x["i"], ib.to(cuda),
+                      cap, x["gate"], nw.to(cuda), out, states, slot, cu, pos, dim ** -0.5, 1e-6, status=status)
+            at = 0
+            for i, lo, hi in entries:
+                got[i][lo:hi] = out[at:at + hi - lo].flatten(1).double().cpu()
+                at += hi - lo
+        run_steps(cuda, lens, portions, step)
+        ops.check_status(status)
+        for a, b in zip(got, want):
+            assert rel(a, b) < 8e-3
