@@ -11,11 +11,13 @@
 // One token per sequence (linear_step_kernel): a CTA per (sequence, head); a thread holds RPT rows x 4 columns of S in registers,
 // so the state is read once and written once (the roofline: HBM, 8 * dim * vdim bytes per head and sequence); gates, normaliser and
 // the gated output norm are in the same kernel.
-// Ragged step, bf16 activations: chunks of 16 tokens on the tensor cores (linear_chunks.cuh).
+// Ragged step, bf16 activations: with exponential gates decay_chunk_kernel (decay_chunks.cuh) where sizes, alignment and prompt lengths
+// allow it, else chunks of 16 tokens on the tensor cores (linear_chunks.cuh).
 // Ragged step, fp32 activations: plain fp32 throughout.  linear_prep_kernel writes q, k and the gates once per token;
 // linear_tokens_kernel walks a sequence's tokens with S in registers (8 row groups x 4 columns per warp, three shuffles for the sum
 // over rows), operands staged TT tokens ahead with cp.async.
 #include "chunk_common.cuh"
+#include "decay_chunks.cuh"
 #include "head_norm.cuh"
 #include "host_util.cuh"
 #include "mini_vllm_b200.h"
@@ -166,6 +168,11 @@ __global__ void __launch_bounds__(512) linear_step_kernel(const LinearParams p, 
 __device__ __forceinline__ void stash_maximum(const LinearParams& p, int s, int h) {
   const int64_t slot = linear_slot(p, s);
   p.m0[s * p.heads + h] = slot < 0 || p.positions[p.cu[s]] == 0 ? 0.f : p.m[slot * p.heads + h];
+}
+
+__global__ void __launch_bounds__(128) stash_maxima_kernel(const LinearParams p) {
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i < p.num_seqs * p.heads && p.cu[i / p.heads + 1] > p.cu[i / p.heads]) stash_maximum(p, i / p.heads, i % p.heads);
 }
 
 // ---- ragged step, fp32: per-token operands ------------------------------------------------------------------------
@@ -337,12 +344,34 @@ static int launch_linear_tokens(const LinearParams& p, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
+// decay_chunk_kernel over whole sequences; the CTAs of the other columns may start after the normaliser's has stored the new maximum
+template <int KB>
+static int launch_mlstm_wide(const LinearParams& p, cudaStream_t st) {
+  CUtensorMap maps[3];
+  const int rc = decay_maps(maps, p.q, p.k, p.v, p.qkv_stride, p.tokens, p.heads, p.dim, p.heads, p.vdim);
+  if (rc != kOk) return rc;
+  stash_maxima_kernel<<<(p.num_seqs * p.heads + 127) / 128, 128, 0, st>>>(p);
+  if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+  DecayChunkParams d{};
+  d.a = static_cast<const __nv_bfloat16*>(p.decay); d.a_stride = p.decay_stride; d.a_bias = p.decay_bias;
+  d.i = static_cast<const __nv_bfloat16*>(p.igate); d.i_stride = p.igate_stride; d.i_bias = p.igate_bias;
+  d.cap = p.cap; d.q_scale = p.q_scale;
+  d.o = p.o; d.nq = p.nq; d.mt = p.mt; d.m0 = p.m0;
+  d.state = p.S; d.n_state = p.n; d.m_state = p.m; d.slots = p.slots; d.num_slots = p.num_slots; d.cu = p.cu; d.positions = p.positions;
+  d.num_seqs = p.num_seqs; d.heads = p.heads; d.per_group = 1; d.n = p.dim; d.vdim = p.vdim; d.vp = p.vp; d.dev_status = p.dev_status;
+  return launch_decay_pass<KB, true, false>(maps, d, p.num_seqs, st);
+}
+
 template <class T, bool EXP>
 static int launch_linear(const LinearParams& p, cudaStream_t st) {
   if (p.cu == nullptr) return launch_linear_step<T, EXP>(p, st);
   if (p.heads > 65535 || p.num_seqs > 65535) return kUnsupportedShape;
   int rc = kUnsupportedShape;
   if constexpr (sizeof(T) == 2) {
+    if (EXP && decay_chunks_fit(p.q, p.k, p.v, p.qkv_stride, p.dim, p.vdim, p.tokens, p.num_seqs, p.heads)) {
+      rc = p.dim == 64 ? launch_mlstm_wide<1>(p, st) : launch_mlstm_wide<2>(p, st);
+      return rc == kOk ? launch_linear_norm<T, EXP>(p, st) : rc;
+    }
     switch (chunk_ks(p.dim)) {
       case 1: rc = launch_linear_chunks<EXP, 1>(p, st); break;
       case 2: rc = launch_linear_chunks<EXP, 2>(p, st); break;
