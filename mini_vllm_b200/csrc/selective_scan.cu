@@ -12,6 +12,9 @@
 // are computed once per (token, channel) into shared memory.
 // One token per sequence (scan_step_kernel): bound by reading and writing the state; no shared memory.
 //
+// 4 sequences of 2,048 tokens, 4,096 channels of 16 states, bf16: 310 us (346 with one state an instruction and five exchanges a token's
+// sum; two channels a lane read less of B and C but left too few warps, 371; 16-token tiles 349; the exponentials alone take 119).
+//
 // Roofline: a ragged step is bound by the special-function unit (channels * N exponentials per token, 16 per clock and SM)
 // or, for few states, by HBM (4 activations of channels elements per token); a decode step by HBM (2 * 4 * channels * N bytes
 // per sequence).
@@ -90,11 +93,10 @@ template <class T, int E> __device__ __forceinline__ Raw<T, E> load_raw(const T*
 // E: channels per thread in the elementwise part (2 where the operands are aligned for it)
 template <class T, int L, int R, int E>
 __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
-  constexpr int CHW = 32 / L, CH = 4 * CHW, NP = 4 * L * R, TT = L <= 8 ? 32 : 16;
-  constexpr int ECH = CH / E, EPT = TT * ECH >= 128 ? TT * ECH / 128 : 1, BPT = TT * 2 * NP / 128;
-  __shared__ __align__(8) float dt_s[TT][CH];
-  __shared__ __align__(8) float du_s[TT][CH];
-  __shared__ __align__(8) float y_s[TT][CH];
+  constexpr int NT = 128, CHW = 32 / L, CH = 4 * CHW, NP = 4 * L * R, TT = L <= 8 ? 32 : 16;
+  constexpr int ECH = CH / E, EPT = TT * ECH >= NT ? TT * ECH / NT : 1, BPT = TT * 2 * NP / NT;
+  __shared__ __align__(16) float2 dtu_s[TT][CH];               // dt, dt u
+  __shared__ __align__(16) float y_s[TT][CH];
   __shared__ __align__(16) float b_s[TT][NP];
   __shared__ __align__(16) float c_s[TT][NP];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane % L;
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
   }
 
   // a thread keeps its E channels throughout and takes every ESTEP-th token of a tile
-  constexpr int ESTEP = 128 / ECH;
+  constexpr int ESTEP = NT / ECH;
   const int ech = tid % ECH * E, etok = tid / ECH;
   const bool ech_ok = c0 + ech < p.channels;
   float bias[E], dskip[E];
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
     pu += TT * p.u_stride; pd += TT * p.dt_stride; pz += TT * p.z_stride;
 #pragma unroll
     for (int k = 0; k < BPT; ++k) {
-      const int e = tid + k * 128, t = t0 + e / (2 * NP), j = e % (2 * NP), nn = j % NP;
+      const int e = tid + k * NT, t = t0 + e / (2 * NP), j = e % (2 * NP), nn = j % NP;
       const T* src = static_cast<const T*>(j < NP ? p.b : p.c);
       rbc[k] = t < n_tok && nn < p.n ? src[(begin + t) * p.bc_stride + nn] : from_f<T>(0.f);
     }
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
     for (int k = 0; k < EPT; ++k) {
       const int tl = etok + k * ESTEP;
       cu_[k] = ru[k]; cz[k] = rz[k];
-      if (TT * ECH < 128 && tl >= TT) continue;
+      if (TT * ECH < NT && tl >= TT) continue;
       const bool in = t0 + tl < n_tok;                       // (a token past the end changes nothing)
       float dt[E], du[E];
 #pragma unroll
@@ -166,27 +168,24 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
         dt[j] = in ? softplus_of<T>(to_f(rdt[k].v[j]) + bias[j]) : 0.f;
         du[j] = dt[j] * to_f(ru[k].v[j]);
       }
-      if constexpr (E == 2) {
-        *reinterpret_cast<float2*>(&dt_s[tl][ech]) = make_float2(dt[0], dt[1]);
-        *reinterpret_cast<float2*>(&du_s[tl][ech]) = make_float2(du[0], du[1]);
-      } else {
-        dt_s[tl][ech] = dt[0];
-        du_s[tl][ech] = du[0];
-      }
+      if constexpr (E == 2) *reinterpret_cast<float4*>(&dtu_s[tl][ech]) = make_float4(dt[0], du[0], dt[1], du[1]);
+      else dtu_s[tl][ech] = make_float2(dt[0], du[0]);
     }
 #pragma unroll
     for (int k = 0; k < BPT; ++k) {
-      const int e = tid + k * 128, tl = e / (2 * NP), j = e % (2 * NP);
+      const int e = tid + k * NT, tl = e / (2 * NP), j = e % (2 * NP);
       if (j < NP) b_s[tl][j] = to_f(rbc[k]); else c_s[tl][j - NP] = to_f(rbc[k]);
     }
     __syncthreads();
     if (t0 + TT < n_tok) request(t0 + TT);
     const int nt = min(TT, n_tok - t0);
-    // four tokens at a time: all operands and exponentials first, so that only the multiply-adds of S are a chain
+    // four tokens at a time: all operands and exponentials first, so that only the multiply-adds of S are a chain; a second four are
+    // requested meanwhile
+#pragma unroll 2
     for (int tb = 0; tb < nt; tb += 4) {
       float dt[4], du[4], acc[4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) { dt[m] = dt_s[tb + m][chl]; du[m] = du_s[tb + m][chl]; acc[m] = 0.f; }
+      for (int m = 0; m < 4; ++m) { const float2 x = dtu_s[tb + m][chl]; dt[m] = x.x; du[m] = x.y; acc[m] = 0.f; }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int n0 = (sub + L * r) * 4;
@@ -196,22 +195,42 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
           bv[m] = *reinterpret_cast<const float4*>(&b_s[tb + m][n0]);
           cv[m] = *reinterpret_cast<const float4*>(&c_s[tb + m][n0]);
         }
+        float(&s)[4] = S[r];
+        if constexpr (sizeof(T) == 2) {           // two states an instruction
+          float2 s01 = make_float2(s[0], s[1]), s23 = make_float2(s[2], s[3]);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          S[r][0] = advance<T>(S[r][0], dt[m] * a[r][0], du[m] * bv[m].x); acc[m] = fmaf(S[r][0], cv[m].x, acc[m]);
-          S[r][1] = advance<T>(S[r][1], dt[m] * a[r][1], du[m] * bv[m].y); acc[m] = fmaf(S[r][1], cv[m].y, acc[m]);
-          S[r][2] = advance<T>(S[r][2], dt[m] * a[r][2], du[m] * bv[m].z); acc[m] = fmaf(S[r][2], cv[m].z, acc[m]);
-          S[r][3] = advance<T>(S[r][3], dt[m] * a[r][3], du[m] * bv[m].w); acc[m] = fmaf(S[r][3], cv[m].w, acc[m]);
+          for (int m = 0; m < 4; ++m) {
+            const float2 t2 = make_float2(dt[m], dt[m]), u2 = make_float2(du[m], du[m]);
+            float2 x = mul_f32x2(t2, make_float2(a[r][0], a[r][1])), y = mul_f32x2(t2, make_float2(a[r][2], a[r][3]));
+            x.x = fast_exp2(x.x); x.y = fast_exp2(x.y); y.x = fast_exp2(y.x); y.y = fast_exp2(y.y);
+            s01 = fma_f32x2(x, s01, mul_f32x2(u2, make_float2(bv[m].x, bv[m].y)));
+            s23 = fma_f32x2(y, s23, mul_f32x2(u2, make_float2(bv[m].z, bv[m].w)));
+            const float2 sum = fma_f32x2(s23, make_float2(cv[m].z, cv[m].w), mul_f32x2(s01, make_float2(cv[m].x, cv[m].y)));
+            acc[m] += sum.x + sum.y;
+          }
+          s[0] = s01.x; s[1] = s01.y; s[2] = s23.x; s[3] = s23.y;
+        } else {
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            s[0] = advance<T>(s[0], dt[m] * a[r][0], du[m] * bv[m].x); acc[m] = fmaf(s[0], cv[m].x, acc[m]);
+            s[1] = advance<T>(s[1], dt[m] * a[r][1], du[m] * bv[m].y); acc[m] = fmaf(s[1], cv[m].y, acc[m]);
+            s[2] = advance<T>(s[2], dt[m] * a[r][2], du[m] * bv[m].z); acc[m] = fmaf(s[2], cv[m].z, acc[m]);
+            s[3] = advance<T>(s[3], dt[m] * a[r][3], du[m] * bv[m].w); acc[m] = fmaf(s[3], cv[m].w, acc[m]);
+          }
         }
       }
+      // halving exchanges: four lanes share four tokens' sums out and end with one each; the channel's other lanes add theirs
+      const bool up1 = lane & 1, up2 = lane & 2;
 #pragma unroll
-      for (int off = 1; off < L; off <<= 1)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], off);
-      if (sub == 0) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m) y_s[tb + m][chl] = acc[m];
+      for (int m = 0; m < 2; ++m) {
+        const float send = up1 ? acc[m] : acc[2 + m];
+        acc[m] = (up1 ? acc[2 + m] : acc[m]) + __shfl_xor_sync(0xffffffffu, send, 1);
       }
+      const float send = up2 ? acc[0] : acc[1];
+      float mine = (up2 ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, send, 2);
+#pragma unroll
+      for (int off = 4; off < L; off <<= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
+      if (sub < 4) y_s[tb + (up1 ? 2 : 0) + (up2 ? 1 : 0)][chl] = mine;
     }
     __syncthreads();
 #pragma unroll
