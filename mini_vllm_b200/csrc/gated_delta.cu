@@ -155,6 +155,178 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const DeltaParams p, in
   }
 }
 
+// The same for many sequences: one CTA per SM walks (sequence, head) pairs while bulk copies bring the states of the next two and take the
+// last one's back, so that HBM waits less for arithmetic.  The sums run in the order of delta_step_kernel.
+//   warps 0..7   arithmetic: thread = 16 rows x 4 columns     warp 8   copies
+// 256 sequences x 16 heads of 128 x 128: 112 us (delta_step_kernel 124; HBM's floor 83).  With 512 threads 126, with two groups of 256 on
+// alternate pairs, which leaves one stage to load ahead, 147: the three stages' round trip of copies bounds it.
+constexpr int kStreamRows = 16, kStreamStages = 3, kStreamThreads = 256, kStreamWarps = kStreamThreads / 32, kStreamBytes = 64 * 1024;
+struct DeltaStreamCfg {
+  static constexpr int VEC = kStreamStages * kStreamBytes;                 // q, k, g, v: 4 x 256 floats
+  static constexpr int RED = VEC + 4 * 256 * 4;                            // two buffers of 4 KB
+  static constexpr int SUMS = RED + 2 * 4096;                              // 3 x 8 floats
+  static constexpr int META = SUMS + 3 * kStreamWarps * 4;                 // per stage: state offset (-1: none), fresh
+  static constexpr int BARS = META + kStreamStages * 16;
+  static constexpr int SMEM = BARS + (2 * kStreamStages + 1) * 8;
+};
+
+template <class T>
+__global__ void __launch_bounds__(kStreamThreads + 32, 1) delta_stream_kernel(const DeltaParams p) {
+  using C = DeltaStreamCfg;
+  extern __shared__ __align__(128) uint8_t smem[];
+  float* q_s = reinterpret_cast<float*>(smem + C::VEC);
+  float *k_s = q_s + 256, *g_s = k_s + 256, *v_s = g_s + 256;
+  float* sums = reinterpret_cast<float*>(smem + C::SUMS);
+  struct Meta { int64_t at; int fresh; int pad; };
+  volatile Meta* meta = reinterpret_cast<volatile Meta*>(smem + C::META);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::BARS);
+  uint64_t* done = full + kStreamStages;
+  volatile int* dead = reinterpret_cast<volatile int*>(done + kStreamStages);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int items = p.num_seqs * p.heads, mine = (items - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  const uint32_t bytes = static_cast<uint32_t>(p.dim) * p.vp * 4;
+  if (tid == 0) {
+    for (int i = 0; i < kStreamStages; ++i) { mbar_init(&full[i], 1); mbar_init(&done[i], kStreamWarps); }
+    *dead = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if (warp == kStreamWarps) {
+    if (lane == 0) {
+      auto load = [&](int i) {
+        const int st = i % kStreamStages, item = blockIdx.x + i * gridDim.x, s = item / p.heads;
+        const int64_t slot = delta_slot(p, s), at = slot < 0 ? -1 : (slot * p.heads + item % p.heads) * static_cast<int64_t>(p.dim) * p.vp;
+        const bool fresh = slot < 0 || p.positions[s] == 0;
+        meta[st].at = at; meta[st].fresh = fresh;
+        if (fresh) mbar_arrive(&full[st]);
+        else {
+          mbar_arrive_expect_tx(&full[st], bytes);
+          bulk_copy(smem_u32(smem + st * kStreamBytes), p.state + at, bytes, smem_u32(&full[st]));
+        }
+      };
+      int loaded = 0;
+      for (; loaded < min(2, mine); ++loaded) load(loaded);
+      for (int i = 0; i < mine; ++i) {
+        if (i + 2 < mine) {                       // into the stage of the state before this one, once it has been read
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          load(i + 2);
+          loaded = i + 3;
+        }
+        const int st = i % kStreamStages;
+        if (!mbar_wait(&done[st], (i / kStreamStages) & 1) || *dead) { *dead = 1; break; }
+        if (meta[st].at >= 0) {
+          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                       ::"l"(p.state + meta[st].at), "r"(smem_u32(smem + st * kStreamBytes)), "r"(bytes) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+      for (int i = max(loaded - kStreamStages, 0); i < loaded; ++i) mbar_wait(&full[i % kStreamStages], (i / kStreamStages) & 1);
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    return;
+  }
+  auto meet = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kStreamThreads) : "memory"); };
+  const int quads = p.vp / 4, row_groups = (p.dim + kStreamRows - 1) / kStreamRows, rg = tid / quads, cq = tid % quads;
+  const bool active = rg < row_groups;
+  // raw operands of the next pair are requested before this one is worked on
+  T rq, rk, ra, rv, rgate, rb;
+  auto request = [&](int i) {
+    const int item = blockIdx.x + i * gridDim.x, s = item / p.heads, h = item % p.heads, kvh = h / (p.heads / p.kv_heads);
+    rq = rk = ra = rv = rgate = from_f<T>(0.f);
+    if (tid < p.dim) {
+      rq = static_cast<const T*>(p.q)[s * p.qkv_stride + static_cast<int64_t>(kvh) * p.dim + tid];
+      rk = static_cast<const T*>(p.k)[s * p.qkv_stride + static_cast<int64_t>(kvh) * p.dim + tid];
+      ra = static_cast<const T*>(p.a)[s * p.a_stride + static_cast<int64_t>(h) * p.dim + tid];
+    }
+    if (tid < p.vdim) {
+      rv = static_cast<const T*>(p.v)[s * p.qkv_stride + static_cast<int64_t>(h) * p.vdim + tid];
+      rgate = static_cast<const T*>(p.gate)[s * p.gate_stride + static_cast<int64_t>(h) * p.vdim + tid];
+    }
+    rb = static_cast<const T*>(p.b)[s * p.b_stride + h];
+  };
+  request(0);
+  for (int i = 0; i < mine; ++i) {
+    const int st = i % kStreamStages, item = blockIdx.x + i * gridDim.x, s = item / p.heads, h = item % p.heads;
+    float* red = reinterpret_cast<float*>(smem + C::RED);
+    float* red2 = red + 1024;
+    float* tile = reinterpret_cast<float*>(smem + st * kStreamBytes);
+    const float qv = to_f(rq), kv = to_f(rk), beta = sigmoid_f(to_f(rb)), gate = to_f(rgate);
+    if (tid < p.dim) {
+      q_s[tid] = qv; k_s[tid] = kv;
+      g_s[tid] = decay_of(to_f(ra), p.dt_bias[h * p.dim + tid], p.exp_a[h]);
+    }
+    v_s[tid] = to_f(rv);
+    float qq = warp_sum(qv * qv), kk = warp_sum(kv * kv);
+    if (lane == 0) { sums[warp] = qq; sums[kStreamWarps + warp] = kk; }
+    if (i + 1 < mine) request(i + 1);
+    if (!*dead && !mbar_wait(&full[st], (i / kStreamStages) & 1)) { *dead = 1; report(p.dev_status, kDevWaitTimeout, i); }
+    const bool fresh = meta[st].fresh, kept = meta[st].at >= 0;
+    float4 S[kStreamRows];
+#pragma unroll
+    for (int r = 0; r < kStreamRows; ++r) {
+      const int row = rg + r * row_groups;
+      S[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (active && !fresh && row < p.dim) S[r] = *reinterpret_cast<const float4*>(tile + row * p.vp + cq * 4);
+    }
+    meet();
+    qq = kk = 0.f;
+#pragma unroll
+    for (int w = 0; w < kStreamWarps; ++w) { qq += sums[w]; kk += sums[kStreamWarps + w]; }
+    const float nq = p.q_scale / sqrtf(qq + kUnitEps), nk = 1.f / sqrtf(kk + kUnitEps);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < kStreamRows; ++r) {
+      const int row = rg + r * row_groups;
+      if (!active || row >= p.dim) continue;
+      const float g = g_s[row], k = k_s[row] * nk;
+      S[r].x *= g; S[r].y *= g; S[r].z *= g; S[r].w *= g;
+      acc.x = fmaf(S[r].x, k, acc.x); acc.y = fmaf(S[r].y, k, acc.y); acc.z = fmaf(S[r].z, k, acc.z); acc.w = fmaf(S[r].w, k, acc.w);
+    }
+    if (active) *reinterpret_cast<float4*>(red + rg * p.vp + cq * 4) = acc;
+    meet();
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) {
+      float4 pr = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int w = 0; w < row_groups; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(red + w * p.vp + cq * 4);
+        pr.x += x.x; pr.y += x.y; pr.z += x.z; pr.w += x.w;
+      }
+      const float4 v = *reinterpret_cast<const float4*>(v_s + cq * 4);
+      const int c = cq * 4;
+      e.x = c + 0 < p.vdim ? beta * (v.x - pr.x) : 0.f; e.y = c + 1 < p.vdim ? beta * (v.y - pr.y) : 0.f;
+      e.z = c + 2 < p.vdim ? beta * (v.z - pr.z) : 0.f; e.w = c + 3 < p.vdim ? beta * (v.w - pr.w) : 0.f;
+    }
+    acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < kStreamRows; ++r) {
+      const int row = rg + r * row_groups;
+      if (!active || row >= p.dim) continue;
+      const float k = k_s[row] * nk, q = q_s[row] * nq;
+      S[r].x = fmaf(k, e.x, S[r].x); S[r].y = fmaf(k, e.y, S[r].y); S[r].z = fmaf(k, e.z, S[r].z); S[r].w = fmaf(k, e.w, S[r].w);
+      acc.x = fmaf(S[r].x, q, acc.x); acc.y = fmaf(S[r].y, q, acc.y); acc.z = fmaf(S[r].z, q, acc.z); acc.w = fmaf(S[r].w, q, acc.w);
+      if (kept) *reinterpret_cast<float4*>(tile + row * p.vp + cq * 4) = S[r];
+    }
+    if (active) *reinterpret_cast<float4*>(red2 + rg * p.vp + cq * 4) = acc;
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&done[st]);
+    meet();
+    float o = 0.f;
+    if (tid < p.vdim)
+      for (int w = 0; w < row_groups; ++w) o += red2[w * p.vp + tid];
+    const float ss = warp_sum(o * o);
+    if (lane == 0) sums[2 * kStreamWarps + warp] = ss;
+    meet();
+    if (tid < p.vdim) {
+      float all = 0.f;
+#pragma unroll
+      for (int w = 0; w < kStreamWarps; ++w) all += sums[2 * kStreamWarps + w];
+      const float r = 1.f / sqrtf(all / static_cast<float>(p.vdim) + p.eps);
+      static_cast<T*>(p.out)[s * p.out_stride + static_cast<int64_t>(h) * p.vdim + tid] = from_f<T>(o * r * p.norm_w[tid] * sigmoid_f(gate) * p.out_scale);
+    }
+  }
+}
+
 // ---- ragged step: per-token operands ------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(256) delta_prep_kernel(const DeltaParams p) {
@@ -306,6 +478,16 @@ template <class T>
 static int launch_step(const DeltaParams& p, cudaStream_t st) {
   const int tile = step_tile_cols(p.vp), tiles = (p.vp + tile - 1) / tile, quads = tile / 4;
   if (p.num_seqs > 65535) return kUnsupportedShape;
+  // at least four states an SM (256 x 16 measured, above), each at least a quarter of the stage it is copied to
+  const int64_t bytes = static_cast<int64_t>(p.dim) * p.vp * 4, items = static_cast<int64_t>(p.num_seqs) * p.heads;
+  if (p.state != nullptr && tiles == 1 && bytes <= kStreamBytes && bytes >= kStreamBytes / 4 && p.vp >= 32 &&
+      (p.dim + kStreamRows - 1) / kStreamRows * quads <= kStreamThreads && items >= 4 * sm_count() && items < (1 << 30)) {
+    struct Tag {};
+    const int rc = opt_in_dynamic_smem<Tag>(reinterpret_cast<const void*>(&delta_stream_kernel<T>), DeltaStreamCfg::SMEM);
+    if (rc != kOk) return rc;
+    delta_stream_kernel<T><<<sm_count(), kStreamThreads + 32, DeltaStreamCfg::SMEM, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+  }
   auto go = [&](auto tag) -> int {
     constexpr int RPT = decltype(tag)::value;
     const int row_groups = (p.dim + RPT - 1) / RPT;
