@@ -141,6 +141,14 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     fence_mbar_init();
   }
   if (warp == 17) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (ones) {                                     // its values, which no copy brings, are there before any role begins: 1 in the first column
+    for (int i = tid; i < 2 * L * 8; i += C::THREADS) {
+      const int row = i >> 3 & (L - 1), j = i & 7;
+      *reinterpret_cast<uint4*>(smem + i / (L * 8) * C::STAGE + C::V + row * 128 + ((j * 16) ^ ((row & 7) << 4))) =
+          make_uint4(j == 0 ? 0x3f80u : 0u, 0u, 0u, 0u);
+    }
+    fence_proxy_async();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -505,13 +513,6 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         S[i][j] = w.x; S[i][j + 1] = w.y; S[i][j + 2] = w.z; S[i][j + 3] = w.w;
       }
       if (!STATES && holds) store_operand(k, S[i]);
-      if (ones) {                                 // the values: 1 in the first column
-#pragma unroll
-        for (int j = 2 * k; j < 2 * k + 2; ++j)
-#pragma unroll
-          for (int st = 0; st < 2; ++st)
-            *reinterpret_cast<uint4*>(smem + st * C::STAGE + C::V + row * 128 + ((j * 16) ^ sw)) = make_uint4(j == 0 ? 0x3f80u : 0u, 0u, 0u, 0u);
-      }
     }
     fence_proxy_async();
     arrive(C::S_READY);

@@ -91,3 +91,51 @@ def test_matrix_memory_edges(cuda, dim, vdim, f_bias, swing):
         ops.check_status(status)
         for a, b in zip(got, want):
             assert rel(a, b) < 8e-3
+
+
+def memory_step(cuda, lens, heads, dim, vdim, f_bias, i_bias, eps, states=None, slots=None, starts=None, seed=0, edit=None):
+    """One ragged step of the matrix memory over new inputs, and what the plain oracle makes of it: outputs, and the state behind each
+    sequence.  ``states`` are changed in place."""
+    g, cap, nw = gen(seed), 15.0, torch.ones(heads * vdim)
+    mk = lambda *s: torch.randn(*s, generator=g).to(BF)
+    seqs = [{"q": mk(t, heads, dim), "k": mk(t, heads, dim), "v": mk(t, heads, vdim), "f": mk(t, heads), "i": mk(t, heads), "gate": mk(t, heads * vdim)}
+            for t in lens]
+    for s in seqs:
+        if edit is not None:
+            edit(s)
+    fb, ib, starts = torch.full((heads,), f_bias), torch.full((heads,), i_bias), starts or [0] * len(lens)
+    capped = lambda x, bias: cap * torch.tanh((x.double() + bias.double()) / cap)
+    want, behind = [], []
+    for j, s in enumerate(seqs):
+        x = {k: v.double() for k, v in s.items()}
+        f, i = torch.nn.functional.logsigmoid(capped(s["f"], fb)), capped(s["i"], ib)
+        has = states is not None and starts[j] > 0 and 0 <= slots[j] < states[0].shape[0]
+        front = lambda h: tuple(z[slots[j], h].double().cpu() for z in states) if has else None
+        runs = [memory.mlstm_memory(x["q"][:, h] * dim ** -0.5, x["k"][:, h], x["v"][:, h], i[:, h], f[:, h], front(h)) for h in range(heads)]
+        o = torch.stack([r[0] for r in runs], dim=1)
+        want.append((o / torch.sqrt((o * o).mean(-1, keepdim=True) + eps)).flatten(1) * torch.sigmoid(x["gate"]))
+        behind.append([torch.stack([r[1][m] for r in runs]) for m in range(3)])
+    x = {k: torch.cat([s[k] for s in seqs]).to(cuda) for k in seqs[0]}
+    q, k, v = torch.cat([x[n].flatten(1) for n in "qkv"], dim=1).split([heads * dim, heads * dim, heads * vdim], dim=1)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=cuda)
+    pos = torch.cat([torch.arange(t) + at for t, at in zip(lens, starts)]).to(cuda)
+    status, out = ops.new_status(cuda), torch.full((sum(lens), heads, vdim), math.nan, dtype=BF, device=cuda)
+    ops.mlstm(q.unflatten(1, (heads, dim)), k.unflatten(1, (heads, dim)), v.unflatten(1, (heads, vdim)), x["f"], fb.to(cuda), x["i"], ib.to(cuda), cap,
+              x["gate"], nw.to(cuda), out, states, None if slots is None else torch.tensor(slots, dtype=torch.int32, device=cuda), cu, pos, dim ** -0.5, eps,
+              status=status)
+    return list(out.flatten(1).double().cpu().split(lens)), want, behind, status
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 64)])
+def test_matrix_memory_goes_on(cuda, dim, vdim):
+    """Prompts behind a state of random values, whose normaliser comes from memory while the first products already run: outputs (an eps that
+    keeps their size visible), memory, normaliser and maximum against the oracle."""
+    heads, lens, slots, g = 16, [130, 5, 128, 257, 64, 200], [3, 6, 0, 1, 7, 4], gen(3)
+    states = tuple(x.to(cuda) for x in (torch.randn(9, heads, dim, vdim, generator=g), torch.randn(9, heads, dim, generator=g), torch.randn(9, heads, generator=g)))
+    torch.empty(64 << 20, device=cuda).zero_()                       # the states are no longer in a cache
+    got, want, behind, status = memory_step(cuda, lens, heads, dim, vdim, 4.0, -1.0, 0.5, states, slots, [7, 9, 0, 3, 1, 2])
+    ops.check_status(status)
+    for j, slot in enumerate(slots):
+        assert rel(got[j], want[j]) < 8e-3
+        # factors of 16 bits, fp32 sums of up to 257 terms
+        assert all(rel(states[m][slot], behind[j][m]) < 3e-5 for m in range(3))
