@@ -85,8 +85,8 @@ __device__ __forceinline__ int by_length(const int32_t* cu, int n, int k) {
   return found;
 }
 
-// The normaliser alone decides the size of an output, so its weights and its state enter with all the bits of fp32: a third bf16 part of
-// its single column, in columns that are free there.
+// The normaliser alone decides the size of an output, and its terms may cancel, so none of it is cut to 16 bits: its part of M is added up
+// in fp32 by the warps that make M, and its weights and its state enter the products with a third bf16 part, in columns that are free there.
 __device__ __forceinline__ uint4 three_parts(float x) {
   const float h = bf16_round(x), m = bf16_round(x - h);
   return make_uint4(pack_bf16(h, m), pack_bf16(x - h - m, 0.f), 0u, 0u);
@@ -141,14 +141,6 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     fence_mbar_init();
   }
   if (warp == 17) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  if (ones) {                                     // its values, which no copy brings, are there before any role begins: 1 in the first column
-    for (int i = tid; i < 2 * L * 8; i += C::THREADS) {
-      const int row = i >> 3 & (L - 1), j = i & 7;
-      *reinterpret_cast<uint4*>(smem + i / (L * 8) * C::STAGE + C::V + row * 128 + ((j * 16) ^ ((row & 7) << 4))) =
-          make_uint4(j == 0 ? 0x3f80u : 0u, 0u, 0u, 0u);
-    }
-    fence_proxy_async();
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -223,6 +215,11 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         ok = wait(C::M_READY + (c & 1), (c >> 1) & 1, 22) && wait(C::V_FULL + (c & 1), (c >> 1) & 1, 23) && (c == 0 || wait(C::Y_FREE, (c - 1) & 1, 24));
         if (!ok) break;
         tc_fence_after();
+        if (ones) {                               // M has been added up; plain arrivals, which hand those sums on
+          mbar_arrive(&bars[C::V_EMPTY + (c & 1)]);
+          mbar_arrive(&bars[C::Y_FULL]);
+          continue;
+        }
         const uint64_t v = umma_desc_sw128(base + (c & 1) * C::STAGE + C::V, 16, 1024);
 #pragma unroll
         for (int part = 0; part < 2; ++part)
@@ -377,7 +374,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 #pragma unroll 1
         for (int j = half * 4; j < half * 4 + 4; ++j) {
           const int at = row * 128 + j * 16;
-          *reinterpret_cast<uint4*>(stage + C::V + at) = zero;
+          if (!ones) *reinterpret_cast<uint4*>(stage + C::V + at) = zero;
 #pragma unroll
           for (int kb = 0; kb < KB; ++kb) *reinterpret_cast<uint4*>(stage + C::K + kb * C::TILE + at) = zero;
           *reinterpret_cast<uint4*>(smem + C::XS + at) = zero;
@@ -422,6 +419,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const uint32_t m_at = lanes + C::T_M + (c & 1) * 128;
         const float* tab = table(c);
         const float r = EXP ? tab[C::X3 + row] : -tab[C::E + row];
+        float sum = 0.f;                          // of the row's part of M (the normaliser's tile)
         // 16 keys at a time, in place: eight columns of high parts, eight of low ones; zeros behind the last key a row can see
 #pragma unroll 1
         for (int b = half; b < 8; b += 2) {
@@ -459,12 +457,18 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 #pragma unroll
             for (int j = 0; j < 16; ++j) g[j] = 0u;
           }
+          if (ones) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum += __uint_as_float(g[j]);
+            continue;
+          }
           uint32_t m[16];
 #pragma unroll
           for (int j = 0; j < 8; ++j) split_pair(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]), m[j], m[8 + j]);
           tmem_st_32x16(m_at + b * 16, m);
         }
         tmem_wait_st();
+        if (ones) reinterpret_cast<float*>(smem + (c & 1) * C::STAGE + C::V)[half * L + row] = sum;      // (where its values would be)
         tc_fence_before();
         arrive(C::M_READY + (c & 1));
         if (c + 1 < n_chunks && !scale_values(c + 1)) break;
@@ -568,7 +572,8 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           if constexpr (EXP) {
             if (ones) {
               const float n0 = __uint_as_float(yi[0]) + (__uint_as_float(yi[1]) + __uint_as_float(yi[2]));
-              if (k == 0 && in) p.nq[t * p.heads + h] = fmaf(n0, f, __uint_as_float(ya[0]));
+              const float* sums = reinterpret_cast<const float*>(smem + (c & 1) * C::STAGE + C::V);
+              if (k == 0 && in) p.nq[t * p.heads + h] = fmaf(n0, f, sums[row] + sums[L + row]);
             } else if (in) {
               float4* o = reinterpret_cast<float4*>(p.o + (t * p.heads + h) * p.vdim + col0 + k * 16);
 #pragma unroll

@@ -139,3 +139,23 @@ def test_matrix_memory_goes_on(cuda, dim, vdim):
         assert rel(got[j], want[j]) < 8e-3
         # factors of 16 bits, fp32 sums of up to 257 terms
         assert all(rel(states[m][slot], behind[j][m]) < 3e-5 for m in range(3))
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 128)])
+def test_a_normaliser_that_all_but_cancels(cuda, dim, vdim):
+    """Two opposite keys, the first a 20,000th weaker by the second's decay: what is left of n . q is a 20,000th of its terms.  Terms of
+    16 bits leave it wrong by 7 %; fp32 weights (four roundings or exponentials of 2^-22 each, at random) by half a per cent."""
+    def edit(s):
+        s["f"][:], s["i"][:] = 0, 0
+        k = s["k"][40].clone()
+        s["k"][:] = 0
+        s["k"][40], s["k"][41] = k * 1000, -k * 1000         # (n . q stays above the floor of its size)
+        s["q"] *= 1000
+    got, want, _, status = memory_step(cuda, [100, 128], 16, dim, vdim, 11.9, 0.0, 1e12, edit=edit)
+    ops.check_status(status)
+    off = []
+    for x, y in zip(got, want):
+        x, y = (z.view(-1, 16, vdim)[41:] for z in (x, y))
+        off.append((x * y).sum(-1) / (y * y).sum(-1) - 1)             # of the size of a head's row: the rounding to bf16 averages out
+    off = float(torch.cat(off).pow(2).mean().sqrt())
+    assert off < 1e-2, off
