@@ -10,8 +10,11 @@
 //                 F_t = sum_{s <= t} f_s; the maximum behind the chunk is F_end - R_end.  The normaliser is one more column of S, whose
 //                 values are 1: a tile of its own.
 //
-// Every exponent that is used is <= 0.  Within 32 tokens of the diagonal 2^{R_t + E_s} is one exponential; further off it is the product of
-// 2^{R_t + rho_b} and 2^{E_s - rho_b}, rho_b the largest E of the 32 keys of block b: three exponentials a row and one a key.
+// Every exponent that is used is <= 0.  Inside a block b of 32 tokens 2^{R_t + E_s} is one exponential; across blocks it is the product of
+// 2^{R_t - R_b} and 2^{E_s + R_b}, R_b that of the last token of the keys' block: three exponentials a row and one a key.
+// F itself, a sum over up to 128 tokens, would round differences that count away.  It is never formed: every token's E and R are measured
+// from the middle of its own block, E + B_b and R - B_b with B_b = F after 16 of the block's tokens, beside the steps from one B to the
+// next, all of them sums over 16 or 32 tokens.
 //
 // A CTA walks one sequence (or segment) for one head and 64 columns of v: products of 128 x 128 and 128 x 64 with fp32 accumulators in
 // tensor memory.  q, k and v are bf16 and enter exactly; M, S and the scaled values enter as bf16 high + low part, so every factor has 16
@@ -55,7 +58,8 @@ struct DecayCfg {
   static constexpr int TILE = kDecayChunk * 128;               // 128 rows of 64 bf16
   static constexpr int Q = 0, K = KB * TILE, V = 2 * KB * TILE, STAGE = (2 * KB + 1) * TILE;
   static constexpr int XS = 2 * STAGE, ST = XS + 2 * TILE, S_PART = KB * 64 * 128, TABLES = ST + 2 * S_PART;
-  static constexpr int E = 0, CS = 128, X3 = 224, M0 = 352, RHO = 353, TABLE = 356;      // in floats
+  // in floats; CS: 2^{E + R_b} (times D); X3: D or R; STEP: m + B_0, B_1 - B_0, B_2 - B_1, B_3 - B_2
+  static constexpr int E = 0, CS = 128, X3 = 224, STEP = 352, TABLE = 356;
   static constexpr int BARS = TABLES + 2 * TABLE * 4;
   // pairs: by chunk parity, where whoever waits could otherwise be two phases behind
   enum { K_FULL = 0, K_EMPTY = 2, Q_FULL = 4, Q_EMPTY = 6, V_FULL = 8, V_EMPTY = 10, TAB = 12, TAB_EMPTY = 14, G_FULL = 16, M_READY = 18,
@@ -283,7 +287,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     };
     request(0);
     for (int c = 0; c < n_chunks; ++c) {
-      float F[4], E[4], D[4], R[4], run = 0.f;
+      float F[4], D[4], E[4], R[4], cs[4], run = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {               // a token past the end changes nothing
         const bool in = c * L + lane * 4 + j < n_tok;
@@ -297,48 +301,55 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         F[j] = run;
       }
       if (c + 1 < n_chunks) request(c + 1);
+      // F - B: sums inside half a block (four lanes), from the middle on or up to it
       float before = run;
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, before, off);
-        if (lane >= off) before += up;
+      for (int off = 1; off < 4; off <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, before, off, 4);
+        if ((lane & 3) >= off) before += up;
       }
-      const float f_end = __shfl_sync(0xffffffffu, before, 31);
+      const float first = __shfl_sync(0xffffffffu, before, (lane & 24) | 3);
+      const float ref = fabsf(first) < INFINITY ? first : 0.f;      // (a gate that is not finite must not reach the tokens in front of it)
       before = __shfl_up_sync(0xffffffffu, before, 1);
-      if (lane == 0) before = 0.f;
-      float top = -INFINITY;
+      before = ((lane & 3) == 0 ? 0.f : before) + (lane & 4 ? first - ref : -ref);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        F[j] += before;
-        E[j] = EXP ? D[j] - F[j] : -F[j];
-        if (EXP) D[j] = p.q_scale;
-        top = fmaxf(top, E[j]);
-        R[j] = EXP ? top : F[j];
-      }
-      float rho = top;                            // of the lane's block: eight lanes
-#pragma unroll
-      for (int off = 1; off < 8; off <<= 1) rho = fmaxf(rho, __shfl_xor_sync(0xffffffffu, rho, off));
+      for (int j = 0; j < 4; ++j) F[j] += before;
+      const float f_end = __shfl_sync(0xffffffffu, F[3], lane | 7), f_last = __shfl_up_sync(0xffffffffu, f_end, 8);      // of the block, of the last
+      float step = lane < 8 ? ref + m : ref + f_last;               // from the last block's B to the own one
       if constexpr (EXP) {
+        float top = -INFINITY;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const float up = __shfl_up_sync(0xffffffffu, top, off);
-          if (lane >= off) top = fmaxf(top, up);
+        for (int j = 0; j < 4; ++j) { E[j] = D[j] - F[j]; top = fmaxf(top, E[j]); R[j] = top; }
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) {
+          const float up = __shfl_up_sync(0xffffffffu, top, off, 8);
+          if ((lane & 7) >= off) top = fmaxf(top, up);
         }
-        float ahead = __shfl_up_sync(0xffffffffu, top, 1);
-        ahead = lane == 0 ? m : fmaxf(ahead, m);
+        // the maximum in front of the block, by way of the blocks before it
+        float ahead = __shfl_sync(0xffffffffu, step, 0);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const float next = fmaxf(ahead, __shfl_sync(0xffffffffu, top, b * 8 + 7)) + __shfl_sync(0xffffffffu, step, b * 8 + 8);
+          if (lane >= b * 8 + 8) ahead = next;
+        }
+        const float up = __shfl_up_sync(0xffffffffu, top, 1);
+        if ((lane & 7) != 0) ahead = fmaxf(ahead, up);
 #pragma unroll
         for (int j = 0; j < 4; ++j) R[j] = -fmaxf(R[j], ahead);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { E[j] = -F[j]; R[j] = F[j]; }
       }
+      const float r_block = __shfl_sync(0xffffffffu, R[3], lane | 7);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cs[j] = fast_exp2(E[j] + r_block) * (EXP ? 1.f : D[j]);
       const bool ok = c < 2 || (wait(C::V_EMPTY + (c & 1), ((c >> 1) - 1) & 1, 35) && wait(C::TAB_EMPTY + (c & 1), ((c >> 1) - 1) & 1, 36));
       if (!__all_sync(0xffffffffu, ok)) break;
       float* tab = table(c);
       *reinterpret_cast<float4*>(tab + C::E + lane * 4) = make_float4(E[0], E[1], E[2], E[3]);
       *reinterpret_cast<float4*>(tab + C::X3 + lane * 4) = EXP ? make_float4(R[0], R[1], R[2], R[3]) : make_float4(D[0], D[1], D[2], D[3]);
-      if (lane < 24)
-        *reinterpret_cast<float4*>(tab + C::CS + lane * 4) = make_float4(fast_exp2(E[0] - rho) * D[0], fast_exp2(E[1] - rho) * D[1],
-                                                                         fast_exp2(E[2] - rho) * D[2], fast_exp2(E[3] - rho) * D[3]);
-      if (lane < 24 && (lane & 7) == 0) tab[C::RHO + (lane >> 3)] = rho;
-      if (lane == 0) tab[C::M0] = m;
+      if (lane < 24) *reinterpret_cast<float4*>(tab + C::CS + lane * 4) = make_float4(cs[0], cs[1], cs[2], cs[3]);
+      if ((lane & 7) == 0) tab[C::STEP + (lane >> 3)] = step;
       arrive(C::TAB + (c & 1));
       if constexpr (EXP) {
         if (ones) {
@@ -348,9 +359,14 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             if (t < n_tok) p.mt[static_cast<int64_t>(begin + t) * p.heads + h] = (F[j] - R[j]) * kFromLog2;
           }
         }
-        m = f_end - __shfl_sync(0xffffffffu, R[3], 31);
+        m = __shfl_sync(0xffffffffu, F[3] - R[3], 31);
       }
-      kept += f_end;
+      if constexpr (STATES) {
+        float sum = f_end;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) sum += __shfl_sync(0xffffffffu, step, b * 8);
+        kept += __shfl_sync(0xffffffffu, sum, 31);
+      }
     }
     if (EXP && ones && lane == 0 && slot >= 0 && !*failed) p.m_state[slot * p.heads + h] = m * kFromLog2;
     if (STATES && blockIdx.x == 0 && lane == 0) p.seg_keep[static_cast<int64_t>(blockIdx.z) * p.heads + h] = fast_exp2(kept);
@@ -359,15 +375,19 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // Loops instead of straight code wherever registers allow it: with everything unrolled the warps of this kernel waited for
     // instructions five times as long as they issued.
     const int quad = warp & 3, row = quad * 32 + lane, half = warp >> 2, sw = (row & 7) << 4;
+    auto r_of = [&](const float* tab, int t) { return EXP ? tab[C::X3 + t] : -tab[C::E + t]; };
     auto scale_values = [&](int c) {
       const int n = c >> 1 & 1;
-      const bool ok = wait(C::TAB + (c & 1), n, 50) && wait(C::V_FULL + (c & 1), n, 51) && wait(C::K_FULL + (c & 1), n, 57) &&
-                      (c == 0 || wait(C::DS_FULL, (c - 1) & 1, 58));
-      if (!__all_sync(0xffffffffu, ok)) return false;
+      if (!__all_sync(0xffffffffu, wait(C::TAB + (c & 1), n, 50))) return false;
       const float* tab = table(c);
       const bool in = c * L + row < n_tok;
-      const float r_end = EXP ? tab[C::X3 + L - 1] : -tab[C::E + L - 1];
-      const float w = fast_exp2(r_end + tab[C::E + row]) * (EXP ? 1.f : tab[C::X3 + row]);
+      // 2^{R_end + E} D, for all but the last block as 2^{R_end - R_b} 2^{E + R_b} D
+      const float4 step = *reinterpret_cast<const float4*>(tab + C::STEP);
+      float w = r_of(tab, L - 1) + (quad == 3 ? tab[C::E + row] : -r_of(tab, quad * 32 + 31));
+      w += quad < 1 ? (step.w + step.z) + step.y : quad < 2 ? step.w + step.z : quad < 3 ? step.w : 0.f;
+      w = fast_exp2(w) * (quad < 3 ? tab[C::CS + row] : EXP ? 1.f : tab[C::X3 + row]);
+      const bool ok = wait(C::V_FULL + (c & 1), n, 51) && wait(C::K_FULL + (c & 1), n, 57) && (c == 0 || wait(C::DS_FULL, (c - 1) & 1, 58));
+      if (!__all_sync(0xffffffffu, ok)) return false;
       uint8_t* stage = smem + (c & 1) * C::STAGE;
       if (!in) {                                  // rows behind the last token may hold anything: zeros
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -414,18 +434,24 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     } else if (going) {
       const float skip = EXP ? 0.f : p.skip[h];
       for (int c = 0; c < n_chunks; ++c) {
+        const float* tab = table(c);              // (waited for with the scaled values)
+        const float r = r_of(tab, row);
+        float rb = r;                             // the row's R, measured from the middle of the keys' block
         if (!__all_sync(0xffffffffu, wait(C::G_FULL + (c & 1), (c >> 1) & 1, 41))) break;
         tc_fence_after();
         const uint32_t m_at = lanes + C::T_M + (c & 1) * 128;
-        const float* tab = table(c);
-        const float r = EXP ? tab[C::X3 + row] : -tab[C::E + row];
         float sum = 0.f;                          // of the row's part of M (the normaliser's tile)
         // 16 keys at a time, in place: eight columns of high parts, eight of low ones; zeros behind the last key a row can see
 #pragma unroll 1
-        for (int b = half; b < 8; b += 2) {
+        for (int b = 6 + half; b >= 0; b -= 2) {
           uint32_t g[16];
           if (b <= 2 * quad + 1) {
             tmem_ld_32x16(m_at + b * 16, g);
+            float f = 0.f;
+            if ((b >> 1) != quad) {
+              rb += tab[C::STEP + (b >> 1) + 1];
+              f = fast_exp2(rb - r_of(tab, (b | 1) * 16 + 15)) * (EXP ? p.q_scale : 1.f);
+            }
             tmem_wait_ld();
             if ((b >> 1) == quad) {
               const int own = row - b * 16;       // the key on the diagonal
@@ -443,7 +469,6 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
                 }
               }
             } else {
-              const float f = fast_exp2(r + tab[C::RHO + (b >> 1)]);
 #pragma unroll
               for (int j = 0; j < 16; j += 4) {
                 const float4 w = *reinterpret_cast<const float4*>(tab + C::CS + b * 16 + j);
@@ -459,7 +484,10 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           }
           if (ones) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sum += __uint_as_float(g[j]);
+            for (int j = 8; j > 0; j >>= 1)
+#pragma unroll
+              for (int i = 0; i < j; ++i) g[i] = __float_as_uint(__uint_as_float(g[i]) + __uint_as_float(g[i + j]));
+            sum += __uint_as_float(g[0]);
             continue;
           }
           uint32_t m[16];
@@ -523,13 +551,19 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     bool ok = true;
     for (int c = 0; c < n_chunks && ok; ++c) {
       const bool more = c + 1 < n_chunks;
-      ok = wait(C::TAB + (c & 1), (c >> 1) & 1, 54) && wait(C::DS_FULL, c & 1, 52);
+      ok = __all_sync(0xffffffffu, wait(C::TAB + (c & 1), (c >> 1) & 1, 54));
+      if (!ok) break;
+      const float* tab = table(c);
+      const float4 step = *reinterpret_cast<const float4*>(tab + C::STEP);      // m + B of the row's block, and of the last
+      const int q = warp & 3;
+      const float own = step.x + (q > 0 ? step.y : 0.f) + (q > 1 ? step.z : 0.f) + (q > 2 ? step.w : 0.f), base = step.x + step.y + step.z + step.w;
+      const float keep = fast_exp2(base + (EXP ? tab[C::X3 + L - 1] : -tab[C::E + L - 1]));
+      const float r = own + (EXP ? tab[C::X3 + row] : -tab[C::E + row]);
+      ok = wait(C::DS_FULL, c & 1, 52);
       if (!STATES) ok = ok && wait(C::INTER, c & 1, 53);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float* tab = table(c);
-      const float m = tab[C::M0], keep = fast_exp2((EXP ? tab[C::X3 + L - 1] : -tab[C::E + L - 1]) + m);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int k = half * 2 + i;
@@ -545,7 +579,6 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
         if (!STATES && more && holds) store_operand(k, S[i]);
       }
-      const float r = EXP ? tab[C::X3 + row] : -tab[C::E + row];
       if (more) {
         fence_proxy_async();
         tc_fence_before();                        // (what the chunk added has been read)
@@ -556,7 +589,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         ok = __all_sync(0xffffffffu, wait(C::Y_FULL, c & 1, 56));
         if (!ok) break;
         tc_fence_after();
-        const float f = fast_exp2(r + m) * (EXP ? p.q_scale : 1.f);
+        const float f = fast_exp2(r) * (EXP ? p.q_scale : 1.f);
         const bool in = c * L + row < n_tok;
         const int64_t t = begin + c * L + row;
         uint8_t* out_s = smem + (c & 1) * C::STAGE + C::Q;

@@ -153,9 +153,76 @@ def test_a_normaliser_that_all_but_cancels(cuda, dim, vdim):
         s["q"] *= 1000
     got, want, _, status = memory_step(cuda, [100, 128], 16, dim, vdim, 11.9, 0.0, 1e12, edit=edit)
     ops.check_status(status)
-    off = []
+    errs = []
     for x, y in zip(got, want):
         x, y = (z.view(-1, 16, vdim)[41:] for z in (x, y))
-        off.append((x * y).sum(-1) / (y * y).sum(-1) - 1)             # of the size of a head's row: the rounding to bf16 averages out
-    off = float(torch.cat(off).pow(2).mean().sqrt())
-    assert off < 1e-2, off
+        errs.append((x * y).sum(-1) / (y * y).sum(-1) - 1)             # of the size of a head's row: the rounding to bf16 averages out
+    err = float(torch.cat(errs).pow(2).mean().sqrt())
+    assert err < 1e-2, err
+
+
+def off(got, want):
+    """2-norm of the difference over that of the result."""
+    got, want = got.double().cpu(), want.double()
+    return float((got - want).norm() / want.norm())
+
+
+def space_step(cuda, lens, heads, groups, n, vdim, dt_bias, a, seed=0, state=None, slots=None, starts=None, edit=None, longest=None):
+    """One ragged step of the state space over new inputs; the inputs, the outputs of each sequence and the status."""
+    g, d = gen(seed), torch.ones(heads)
+    seqs = space_inputs(g, lens, heads, groups, n, vdim)
+    for s in seqs:
+        if edit is not None:
+            edit(s)
+    bias = torch.full((heads,), dt_bias)
+    x, b, c = torch.cat([torch.cat([s[k].flatten(1) for k in "xbc"], dim=1) for s in seqs]).to(cuda).split([heads * vdim, groups * n, groups * n], dim=1)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=cuda)
+    pos = torch.cat([torch.arange(t) + at for t, at in zip(lens, starts or [0] * len(lens))]).to(cuda)
+    status, out = ops.new_status(cuda), torch.full((sum(lens), heads, vdim), math.nan, dtype=BF, device=cuda)
+    ops.state_space(x.unflatten(1, (heads, vdim)), b.unflatten(1, (groups, n)), c.unflatten(1, (groups, n)), torch.cat([s["dt"] for s in seqs]).to(cuda),
+                    *(z.float().to(cuda) for z in (bias, a / math.log(2.0), d)), out, state,
+                    None if slots is None else torch.tensor(slots, dtype=torch.int32, device=cuda), cu, pos, longest=max(lens) if longest is None else longest,
+                    status=status)
+    return seqs, list(out.cpu().split(lens)), status
+
+
+def space_walk(s, bias, a, state=None):
+    """The recurrence in 64 bits: outputs and the state behind it, from ``state`` [heads, n, vdim] or zero."""
+    x, heads = {k: v.double() for k, v in s.items()}, s["x"].shape[1]
+    b, c = (x[k].repeat_interleave(heads // x[k].shape[1], dim=1) for k in "bc")
+    dt, ys = torch.nn.functional.softplus(x["dt"] + bias), []
+    S = torch.zeros(heads, b.shape[2], x["x"].shape[2], dtype=torch.float64) if state is None else state.double().cpu()
+    for t in range(dt.shape[0]):
+        S = S * torch.exp(a.double() * dt[t])[:, None, None] + (dt[t][:, None] * b[t])[:, :, None] * x["x"][t][:, None, :]
+        ys.append((S * c[t][:, :, None]).sum(1) + x["x"][t])
+    return torch.stack(ys), S
+
+
+@pytest.mark.parametrize("n,vdim", [(64, 64), (128, 128)])
+def test_weak_decays_behind_strong_ones(cuda, n, vdim):
+    """32 tokens that forget little at the end of chunks whose other tokens forget nearly everything: the sums of the decays are hundreds of
+    times the differences that count.  A weight enters a product in two bf16 parts, which leave up to 2^-18 of it; the step's logarithm of
+    1 + e^-3 is rounded at 2^-24 of 1, 1.2e-6 of the step, and 32 equal steps times 2 make an exponent of 3.1 of it."""
+    def edit(s):
+        s["dt"][:96], s["dt"][96:128] = 6, -3
+    state = torch.zeros(1, 4, n, vdim, device=cuda)
+    a = -torch.tensor([1.0, 1.3, 0.7, 2.0])
+    seqs, got, status = space_step(cuda, [128], 4, 2, n, vdim, 0.0, a, n, state, [0], edit=edit)
+    ops.check_status(status)
+    y, S = space_walk(seqs[0], 0.0, a)
+    assert off(got[0], y) < 4e-3
+    err = off(state[0], S)
+    assert err < 9e-6, err
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128)])
+def test_weak_forget_gates_behind_strong_ones(cuda, dim, vdim):
+    """The same of the matrix memory; its gates' functions are those of CUDA, exact to a few ulps."""
+    def edit(s):
+        s["f"][:96], s["f"][96:128], s["i"] = -40, 8, s["i"] * 0.1
+    states = tuple(torch.zeros(*s, device=cuda) for s in ((1, 3, dim, vdim), (1, 3, dim), (1, 3)))
+    got, want, behind, status = memory_step(cuda, [128], 3, dim, vdim, 0.0, 0.0, 0.5, states, [0], edit=edit)
+    ops.check_status(status)
+    assert off(got[0], want[0]) < 4e-3
+    errs = [off(x[0], y) for x, y in zip(states, behind[0])]
+    assert max(errs[:2]) < 2 ** -18, errs
