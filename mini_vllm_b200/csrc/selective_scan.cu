@@ -13,7 +13,8 @@
 // One token per sequence (scan_step_kernel): bound by reading and writing the state; no shared memory.
 //
 // 4 sequences of 2,048 tokens, 4,096 channels of 16 states, bf16: 310 us (346 with one state an instruction and five exchanges a token's
-// sum; two channels a lane read less of B and C but left too few warps, 371; 16-token tiles 349; the exponentials alone take 119).
+// sum; two channels a lane read less of B and C but left too few warps, 371; 16-token tiles 349; at 16 exponentials per clock and SM the
+// special function unit alone needs 119).
 //
 // Roofline: a ragged step is bound by the special-function unit (channels * N exponentials per token, 16 per clock and SM)
 // or, for few states, by HBM (4 activations of channels elements per token); a decode step by HBM (2 * 4 * channels * N bytes
@@ -180,8 +181,9 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
     if (t0 + TT < n_tok) request(t0 + TT);
     const int nt = min(TT, n_tok - t0);
     // four tokens at a time: all operands and exponentials first, so that only the multiply-adds of S are a chain; a second four are
-    // requested meanwhile
-#pragma unroll 2
+    // requested meanwhile where that is faster: 1.10 to 1.35 times up to 32 states in bf16, but 0.9 times with 256 in fp32
+    constexpr int AHEAD = sizeof(T) == 2 && L <= 8 ? 2 : 1;
+#pragma unroll AHEAD
     for (int tb = 0; tb < nt; tb += 4) {
       float dt[4], du[4], acc[4];
 #pragma unroll
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(128) scan_tokens_kernel(const ScanParams p) {
           cv[m] = *reinterpret_cast<const float4*>(&c_s[tb + m][n0]);
         }
         float(&s)[4] = S[r];
-        if constexpr (sizeof(T) == 2) {           // two states an instruction
+        if constexpr (sizeof(T) == 2 && L <= 16) {             // two states an instruction (64 sequences of 3 tokens, 128 states: 0.95 times)
           float2 s01 = make_float2(s[0], s[1]), s23 = make_float2(s[2], s[3]);
 #pragma unroll
           for (int m = 0; m < 4; ++m) {
