@@ -18,11 +18,12 @@
 //
 // A CTA walks one sequence (or segment) for one head and 64 columns of v: products of 128 x 128 and 128 x 64 with fp32 accumulators in
 // tensor memory.  q, k and v are bf16 and enter exactly; M, S and the scaled values enter as bf16 high + low part, so every factor has 16
-// significant bits; S itself stays in fp32 registers.
+// significant bits; S itself stays in fp32 registers.  The matrix memory's scaled values have a third part: its chunks of 16 tokens carried
+// every sixteenth weight, the largest, exactly, and with two parts a state was 1.18 times as far from 64 bits as with those (2.05e-6).
 //   warps 0..7    M, which goes to tensor memory as an operand, and the scaled values of the next chunk; rows of 32 by warp mod 4, two
 //                 warps a row
 //   warps 8..15   S and the outputs, shared out alike
-//   warp 16       TMA: q, k and v of the next chunk while this one is worked on (two stages of 80 KB)
+//   warp 16       TMA: q, k and v of the next chunk while this one is worked on (two stages; one of q where the third part takes its place)
 //   warps 17, 19  tcgen05.mma
 //   warp 18       gates of the next chunk
 // What bounds it: 2,048 tensor-core cycles per 128 tokens, head and 64 columns (N = 128), about 3,200 with their operands' way through
@@ -53,11 +54,12 @@ struct DecayChunkParams {
 // a descriptor that starts `units` of 16 bytes further on (its address is in the low word, and stays there)
 __device__ __forceinline__ uint64_t desc_plus(uint64_t d, uint32_t units) { return (d & 0xffffffff00000000ull) | (static_cast<uint32_t>(d) + units); }
 
-template <int KB>                                              // 64 KB state channels
+template <int KB, bool EXP>                                    // 64 KB state channels
 struct DecayCfg {
   static constexpr int TILE = kDecayChunk * 128;               // 128 rows of 64 bf16
-  static constexpr int Q = 0, K = KB * TILE, V = 2 * KB * TILE, STAGE = (2 * KB + 1) * TILE;
-  static constexpr int XS = 2 * STAGE, ST = XS + 2 * TILE, S_PART = KB * 64 * 128, TABLES = ST + 2 * S_PART;
+  static constexpr int K = EXP ? 0 : KB * TILE, V = K + KB * TILE, STAGE = V + TILE, PARTS = EXP ? 3 : 2;
+  static constexpr int Q_STAGES = EXP ? 1 : 2, Q = EXP ? 2 * STAGE : 0, Q_TILE = EXP ? 0 : STAGE;
+  static constexpr int XS = 2 * STAGE + (EXP ? KB * TILE : 0), ST = XS + PARTS * TILE, S_PART = KB * 64 * 128, TABLES = ST + 2 * S_PART;
   // in floats; CS: 2^{E + R_b} (times D); X3: D or R; STEP: m + B_0, B_1 - B_0, B_2 - B_1, B_3 - B_2
   static constexpr int E = 0, CS = 128, X3 = 224, STEP = 352, TABLE = 356;
   static constexpr int BARS = TABLES + 2 * TABLE * 4;
@@ -68,6 +70,8 @@ struct DecayCfg {
   static constexpr int THREADS = 20 * 32;
   static constexpr int T_M = 0, T_YI = 256, T_DS = 320, T_YA = 448;                      // tensor memory columns; two buffers of M
   static_assert(SMEM <= 232448, "");
+  static __device__ __forceinline__ int q_stage(int c) { return c & (Q_STAGES - 1); }      // of chunk c, and the parity of its barriers
+  static __device__ __forceinline__ uint32_t q_parity(int c) { return (c / Q_STAGES) & 1; }
 };
 
 // The sequence that is k-th in length, the longest first (n <= 64): CTAs start in about this order, so that no long one starts last.
@@ -96,12 +100,28 @@ __device__ __forceinline__ uint4 three_parts(float x) {
   return make_uint4(pack_bf16(h, m), pack_bf16(x - h - m, 0.f), 0u, 0u);
 }
 
+// a pair of values times w as bf16 high and low parts, and what those two leave
+template <bool THREE>
+__device__ __forceinline__ void split_value(uint32_t v, float w, uint32_t& hi, uint32_t& lo, uint32_t& third) {
+  const float x = bf16_lo(v) * w, y = bf16_hi(v) * w;
+  if constexpr (THREE) {
+    const float2 minus = make_float2(-1.f, -1.f);
+    hi = pack_bf16(x, y);
+    const float2 rest = fma_f32x2(make_float2(bf16_lo(hi), bf16_hi(hi)), minus, make_float2(x, y));      // (exact)
+    lo = pack_bf16(rest.x, rest.y);
+    const float2 last = fma_f32x2(make_float2(bf16_lo(lo), bf16_hi(lo)), minus, rest);
+    third = pack_bf16(last.x, last.y);
+  } else {
+    split_pair(x, y, hi, lo);
+  }
+}
+
 // EXP: matrix memory.  STATES: only what a segment adds to the state, and what it leaves of the one before, is wanted.
 template <int KB, bool EXP, bool STATES>
-__global__ void __launch_bounds__(DecayCfg<KB>::THREADS, 1)
+__global__ void __launch_bounds__(DecayCfg<KB, EXP>::THREADS, 1)
 decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                    const DecayChunkParams p) {
-  using C = DecayCfg<KB>;
+  using C = DecayCfg<KB, EXP>;
   constexpr int L = kDecayChunk;
   constexpr float kToLog2 = 1.4426950408889634f, kFromLog2 = 0.6931471805599453f;
   extern __shared__ __align__(1024) uint8_t decay_smem[];      // (128-byte swizzle: 1024-byte boundaries)
@@ -138,8 +158,8 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   if (tid == 0) {
     for (int b = 0; b < C::NUM_BARS; ++b) {
       const int kind = b < C::XS_READY ? b & ~1 : b;
-      const bool by_eight = kind == C::M_READY || kind == C::TAB_EMPTY || kind == C::Q_EMPTY || b == C::XS_READY || b == C::S_READY || b == C::Y_FREE;
-      mbar_init(&bars[b], by_eight ? 8 : kind == C::K_EMPTY && !STATES ? 2 : 1);
+      const bool by_eight = kind == C::M_READY || kind == C::TAB_EMPTY || (kind == C::Q_EMPTY && !EXP) || b == C::XS_READY || b == C::S_READY || b == C::Y_FREE;
+      mbar_init(&bars[b], by_eight ? 8 : (kind == C::K_EMPTY && !STATES) || kind == C::Q_EMPTY ? 2 : 1);
     }
     *failed = 0;
     fence_mbar_init();
@@ -182,16 +202,17 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
         vs = c + 1;
         if (STATES) continue;
-        if (c >= 2 && !wait(C::Q_EMPTY + st, before, 12)) break;
-        mbar_arrive_expect_tx(&bars[C::Q_FULL + st], KB * C::TILE);
+        const int qst = C::q_stage(c);
+        if (c >= C::Q_STAGES && !wait(C::Q_EMPTY + qst, C::q_parity(c - C::Q_STAGES), 12)) break;
+        mbar_arrive_expect_tx(&bars[C::Q_FULL + qst], KB * C::TILE);
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) tma_load_3d(base + C::Q + kb * C::TILE, &q_map, &bars[C::Q_FULL + st], kb * 64, group, row);
+        for (int kb = 0; kb < KB; ++kb) tma_load_3d(smem + C::Q + qst * C::Q_TILE + kb * C::TILE, &q_map, &bars[C::Q_FULL + qst], kb * 64, group, row);
         qs = c + 1;
       }
       // no copy may be in flight when the CTA ends
       for (int c = max(ks - 2, 0); c < ks; ++c) mbar_wait(&bars[C::K_FULL + (c & 1)], (c >> 1) & 1);
       for (int c = max(vs - 2, 0); c < vs; ++c) mbar_wait(&bars[C::V_FULL + (c & 1)], (c >> 1) & 1);
-      for (int c = max(qs - 2, 0); c < qs; ++c) mbar_wait(&bars[C::Q_FULL + (c & 1)], (c >> 1) & 1);
+      for (int c = max(qs - C::Q_STAGES, 0); c < qs; ++c) mbar_wait(&bars[C::Q_FULL + C::q_stage(c)], C::q_parity(c));
     }
     __syncwarp();
   } else if (warp == 17) {
@@ -201,8 +222,8 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       const uint32_t base = smem_u32(smem);
       auto scores = [&](int c) {                  // over an older M, whose product has been issued
         const uint32_t stage = base + (c & 1) * C::STAGE;
-        const uint64_t q = umma_desc_sw128(stage + C::Q, 16, 1024), k = umma_desc_sw128(stage + C::K, 16, 1024);
-        if (!wait(C::K_FULL + (c & 1), (c >> 1) & 1, 20) || !wait(C::Q_FULL + (c & 1), (c >> 1) & 1, 21)) return false;
+        const uint64_t q = umma_desc_sw128(base + C::Q + C::q_stage(c) * C::Q_TILE, 16, 1024), k = umma_desc_sw128(stage + C::K, 16, 1024);
+        if (!wait(C::K_FULL + (c & 1), (c >> 1) & 1, 20) || !wait(C::Q_FULL + C::q_stage(c), C::q_parity(c), 21)) return false;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4 * KB; ++ks) {
@@ -210,6 +231,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           umma_bf16_ss(tmem + C::T_M + (c & 1) * 128, desc_plus(q, o), desc_plus(k, o), ID_G, ks > 0);
         }
         umma_commit(&bars[C::K_EMPTY + (c & 1)]);
+        if (EXP) umma_commit(&bars[C::Q_EMPTY]);
         umma_commit(&bars[C::G_FULL + (c & 1)]);
         return true;
       };
@@ -239,10 +261,11 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // ============================ tcgen05.mma: what the chunk adds to S, q S0 ==========================
     // (a second thread: one alone would be busy issuing for longer than the products take)
     if (lane == 0) {
-      constexpr uint32_t ID_DS = umma_idesc_bf16(128, 128, true, true), ID_Y = umma_idesc_bf16(128, 64, false, true);
+      constexpr uint32_t ID_DS = umma_idesc_bf16(128, 128, true, true), ID_DT = umma_idesc_bf16(128, 64, true, true), ID_Y = umma_idesc_bf16(128, 64, false, true);
       const uint32_t base = smem_u32(smem);
-      // the scaled values' high and low parts side by side: one product of 128 columns for both
+      // the scaled values' high and low parts side by side: one product of 128 columns for both; a third part on top of the low ones
       const uint64_t xs = umma_desc_sw128(base + C::XS, C::TILE, 1024), sd = umma_desc_sw128(base + C::ST, 16, 1024);
+      const uint64_t xt = umma_desc_sw128(base + C::XS + 2 * C::TILE, 16, 1024);
       for (int c = 0; c < n_chunks; ++c) {
         const uint32_t stage = base + (c & 1) * C::STAGE;
         // k; scaled values; S, and what the last chunk added has been read
@@ -252,21 +275,26 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const uint64_t kt = umma_desc_sw128(stage + C::K, KB == 2 ? C::TILE : 0, 1024);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) umma_bf16_ss(tmem + C::T_DS, desc_plus(kt, ks * 2048 >> 4), desc_plus(xs, ks * 2048 >> 4), ID_DS, ks > 0);
+        if (EXP && !ones) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) umma_bf16_ss(tmem + C::T_DS + 64, desc_plus(kt, ks * 2048 >> 4), desc_plus(xt, ks * 2048 >> 4), ID_DT, true);
+        }
         umma_commit(&bars[C::DS_FULL]);
         umma_commit(&bars[C::K_EMPTY + (c & 1)]);
         if (STATES) {
           umma_commit(&bars[C::V_EMPTY + (c & 1)]);
           continue;
         }
-        if (!wait(C::Q_FULL + (c & 1), (c >> 1) & 1, 33) || (c > 0 && !wait(C::Y_FREE, (c - 1) & 1, 34))) break;
+        if (!wait(C::Q_FULL + C::q_stage(c), C::q_parity(c), 33) || (c > 0 && !wait(C::Y_FREE, (c - 1) & 1, 34))) break;
         tc_fence_after();
-        const uint64_t q = umma_desc_sw128(stage + C::Q, 16, 1024);
+        const uint64_t q = umma_desc_sw128(base + C::Q + C::q_stage(c) * C::Q_TILE, 16, 1024);
 #pragma unroll
         for (int part = 0; part < 2; ++part)
 #pragma unroll
           for (int ks = 0; ks < 4 * KB; ++ks)
             umma_bf16_ss(tmem + C::T_YI, desc_plus(q, (ks / 4 * C::TILE + ks % 4 * 32) >> 4), desc_plus(sd, (part * C::S_PART + ks * 2048) >> 4), ID_Y,
                          part > 0 || ks > 0);
+        if (EXP) umma_commit(&bars[C::Q_EMPTY]);
         umma_commit(&bars[C::INTER]);
       }
     }
@@ -397,8 +425,8 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           if (!ones) *reinterpret_cast<uint4*>(stage + C::V + at) = zero;
 #pragma unroll
           for (int kb = 0; kb < KB; ++kb) *reinterpret_cast<uint4*>(stage + C::K + kb * C::TILE + at) = zero;
-          *reinterpret_cast<uint4*>(smem + C::XS + at) = zero;
-          *reinterpret_cast<uint4*>(smem + C::XS + C::TILE + at) = zero;
+#pragma unroll
+          for (int part = 0; part < C::PARTS; ++part) *reinterpret_cast<uint4*>(smem + C::XS + part * C::TILE + at) = zero;
         }
       } else if (ones) {
 #pragma unroll 1
@@ -415,10 +443,11 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           for (int i = 0; i < 2; ++i) x[i] = *reinterpret_cast<const uint4*>(stage + C::V + row * 128 + (((j + i) * 16) ^ sw));
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            uint4 hi, lo;
-            split_pair(bf16_lo(x[i].x) * w, bf16_hi(x[i].x) * w, hi.x, lo.x); split_pair(bf16_lo(x[i].y) * w, bf16_hi(x[i].y) * w, hi.y, lo.y);
-            split_pair(bf16_lo(x[i].z) * w, bf16_hi(x[i].z) * w, hi.z, lo.z); split_pair(bf16_lo(x[i].w) * w, bf16_hi(x[i].w) * w, hi.w, lo.w);
+            uint4 hi, lo, third = make_uint4(0u, 0u, 0u, 0u);
+            split_value<EXP>(x[i].x, w, hi.x, lo.x, third.x); split_value<EXP>(x[i].y, w, hi.y, lo.y, third.y);
+            split_value<EXP>(x[i].z, w, hi.z, lo.z, third.z); split_value<EXP>(x[i].w, w, hi.w, lo.w, third.w);
             uint8_t* at = smem + C::XS + row * 128 + (((j + i) * 16) ^ sw);
+            if (EXP) *reinterpret_cast<uint4*>(at + 2 * C::TILE) = third;
             *reinterpret_cast<uint4*>(at) = hi;
             *reinterpret_cast<uint4*>(at + C::TILE) = lo;
           }
@@ -592,7 +621,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const float f = fast_exp2(r) * (EXP ? p.q_scale : 1.f);
         const bool in = c * L + row < n_tok;
         const int64_t t = begin + c * L + row;
-        uint8_t* out_s = smem + (c & 1) * C::STAGE + C::Q;
+        uint8_t* out_s = smem + C::Q + C::q_stage(c) * C::Q_TILE;
 #pragma unroll 1
         for (int k = half * 2; k < half * 2 + 2; ++k) {
           uint32_t yi[16], ya[16];
@@ -634,7 +663,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           }
           fence_proxy_async();
         }
-        arrive(C::Q_EMPTY + (c & 1));
+        if (!EXP) arrive(C::Q_EMPTY + (c & 1));
       }
     }
     ok = __all_sync(0xffffffffu, ok && *failed == 0);
@@ -678,9 +707,9 @@ template <int KB, bool EXP, bool STATES>
 static int launch_decay_pass(const CUtensorMap (&maps)[3], const DecayChunkParams& p, unsigned z, cudaStream_t st) {
   struct Tag {};
   auto kernel = &decay_chunk_kernel<KB, EXP, STATES>;
-  const int rc = opt_in_dynamic_smem<Tag>(reinterpret_cast<const void*>(kernel), DecayCfg<KB>::SMEM);
+  const int rc = opt_in_dynamic_smem<Tag>(reinterpret_cast<const void*>(kernel), DecayCfg<KB, EXP>::SMEM);
   if (rc != kOk) return rc;
-  kernel<<<dim3(p.vdim / 64 + (EXP ? 1 : 0), p.heads, z), DecayCfg<KB>::THREADS, DecayCfg<KB>::SMEM, st>>>(maps[0], maps[1], maps[2], p);
+  kernel<<<dim3(p.vdim / 64 + (EXP ? 1 : 0), p.heads, z), DecayCfg<KB, EXP>::THREADS, DecayCfg<KB, EXP>::SMEM, st>>>(maps[0], maps[1], maps[2], p);
   return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 

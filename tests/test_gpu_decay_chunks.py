@@ -226,3 +226,14 @@ def test_weak_forget_gates_behind_strong_ones(cuda, dim, vdim):
     assert off(got[0], want[0]) < 4e-3
     errs = [off(x[0], y) for x, y in zip(states, behind[0])]
     assert max(errs[:2]) < 2 ** -18, errs
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
+def test_memory_keeps_fp32(cuda, dim, vdim):
+    """The memory behind a prompt is as far from 64 bits as fp32 weights leave it (a handful of roundings and exponentials of 2^-23 each, at
+    random): the values enter in three bf16 parts; two alone leave 2e-6."""
+    states = tuple(torch.zeros(*s, device=cuda) for s in ((1, 3, dim, vdim), (1, 3, dim), (1, 3)))
+    got, want, behind, status = memory_step(cuda, [520], 3, dim, vdim, 3.0, -1.0, 0.5, states, [0], seed=2)
+    ops.check_status(status)
+    errs = [off(x[0], y) for x, y in zip(states, behind[0])]
+    assert off(got[0], want[0]) < 4e-3 and max(errs) < 8e-7, errs
