@@ -478,9 +478,11 @@ template <class T>
 static int launch_step(const DeltaParams& p, cudaStream_t st) {
   const int tile = step_tile_cols(p.vp), tiles = (p.vp + tile - 1) / tile, quads = tile / 4;
   if (p.num_seqs > 65535) return kUnsupportedShape;
-  // at least four states an SM (256 x 16 measured, above), each at least a quarter of the stage it is copied to
+  // at least four states an SM, each at least three quarters of the stage it is copied to: with smaller ones two loads ahead are too little in
+  // flight.  delta_step_kernel took, at 4 / 8 / 16 / 60 states an SM (148 SMs), 1.16 / 1.16 / 1.13 / 1.13 times as long with 64 KB (128 x 128),
+  // 1.04 / 1.07 / 1.09 / 1.05 with 48 KB (96 x 128), but 1.09 / 0.92 / 0.87 / 0.78 with 40 KB (80 x 128) and 0.67 / 0.59 / 0.48 / 0.40 with 16 KB
   const int64_t bytes = static_cast<int64_t>(p.dim) * p.vp * 4, items = static_cast<int64_t>(p.num_seqs) * p.heads;
-  if (p.state != nullptr && tiles == 1 && bytes <= kStreamBytes && bytes >= kStreamBytes / 4 && p.vp >= 32 &&
+  if (p.state != nullptr && tiles == 1 && bytes <= kStreamBytes && bytes >= kStreamBytes / 4 * 3 && p.vp >= 32 &&
       (p.dim + kStreamRows - 1) / kStreamRows * quads <= kStreamThreads && items >= 4 * sm_count() && items < (1 << 30)) {
     struct Tag {};
     const int rc = opt_in_dynamic_smem<Tag>(reinterpret_cast<const void*>(&delta_stream_kernel<T>), DeltaStreamCfg::SMEM);

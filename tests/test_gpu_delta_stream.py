@@ -12,7 +12,7 @@ BF, F32 = torch.bfloat16, torch.float32
 
 @pytest.mark.parametrize("dtype", [BF, F32])
 @pytest.mark.parametrize("heads,kv,dim,vdim,seqs", [(16, 16, 128, 128, 40), (4, 2, 128, 128, 257), (8, 8, 64, 64, 75), (6, 3, 100, 90, 100), (8, 8, 256, 64, 76),
-                                                    (5, 1, 40, 127, 150)])
+                                                    (5, 1, 40, 127, 150), (6, 3, 100, 126, 100), (16, 4, 96, 128, 37), (3, 3, 250, 50, 201)])
 def test_many_states(cuda, dtype, heads, kv, dim, vdim, seqs):
     g, small = gen(dim + vdim), 1
     mk = lambda *s: torch.randn(*s, generator=g).to(dtype).to(cuda)
