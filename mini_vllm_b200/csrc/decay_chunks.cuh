@@ -74,23 +74,16 @@ struct DecayCfg {
   static __device__ __forceinline__ uint32_t q_parity(int c) { return (c / Q_STAGES) & 1; }
 };
 
-// The sequence that is k-th in length, the longest first (n <= 64): CTAs start in about this order, so that no long one starts last.
-// A warp at a time; each for itself.
+// The sequence that is k-th in length, the longest first (n <= 32): CTAs start in about this order, so that no long one starts last.
+// With more sequences there are waves enough; ranking 64 took longer than it gave (single chunks: 0.73 instead of 0.92 times the speed).
 __device__ __forceinline__ int by_length(const int32_t* cu, int n, int k) {
-  const int lane = threadIdx.x & 31;
-  int found = 0;
-#pragma unroll 1
-  for (int i = lane; i - lane < n; i += 32) {
-    const int mine = i < n ? cu[i + 1] - cu[i] : -1;
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const int other = cu[j + 1] - cu[j];
-      rank += other > mine || (other == mine && j < i);
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, i < n && rank == k);
-    if (hit) found = i - lane + __ffs(hit) - 1;
+  const int lane = threadIdx.x & 31, mine = lane < n ? cu[lane + 1] - cu[lane] : -1;
+  int rank = 0;
+  for (int j = 0; j < n; ++j) {
+    const int other = __shfl_sync(0xffffffffu, mine, j);
+    rank += other > mine || (other == mine && j < lane);
   }
-  return found;
+  return __ffs(__ballot_sync(0xffffffffu, lane < n && rank == k)) - 1;
 }
 
 // The normaliser alone decides the size of an output, and its terms may cancel, so none of it is cut to 16 bits: its part of M is added up
@@ -132,7 +125,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
   int s = blockIdx.z, begin, end;
   if (p.seg == 0) {
-    if (p.num_seqs <= 64) s = by_length(p.cu, p.num_seqs, s);
+    if (p.num_seqs <= 32) s = by_length(p.cu, p.num_seqs, s);
     begin = p.cu[s]; end = p.cu[s + 1];
   } else {                                        // the sequence and the rows of a segment slot
     int lo = 0, hi = p.num_seqs;
@@ -695,12 +688,23 @@ static int decay_maps(CUtensorMap (&maps)[3], const void* q, const void* k, cons
   return rc;
 }
 // what the kernel takes: 64 or 128 state channels, whole 64-column tiles, rows that TMA can read
-// - and prompts that fill its chunks: on 148 SMs, 16 prompts of 16 / 64 / 100 / 256 tokens took 80 / 72 / 70 / 91 us here and 50 / 48 /
-// 71 / 128 us in chunks of 64 (state space, 64 heads of 64 x 128), 80 / 77 / 79 / 117 and 40 / 56 / 85 / 169 us in chunks of 16 (matrix
-// memory, 16 heads of 128 x 128).  While every tile has an SM to itself the two are equal for short prompts, and long ones win.
-static inline bool decay_chunks_fit(const void* q, const void* k, const void* v, int64_t stride, int n, int vdim, int tokens, int num_seqs, int heads) {
-  const bool filled = tokens >= 96ll * num_seqs || static_cast<int64_t>(num_seqs) * heads * (vdim / 64) <= sm_count();
-  return filled && (n == 64 || n == 128) && vdim % 64 == 0 && stride > 0 && stride % 8 == 0 && is_aligned(q, 16) && is_aligned(k, 16) && is_aligned(v, 16);
+static inline bool decay_chunks_take(int n, int vdim) { return (n == 64 || n == 128) && vdim % 64 == 0; }
+static inline bool decay_chunks_read(const void* q, const void* k, const void* v, int64_t stride) {
+  return stride > 0 && stride % 8 == 0 && is_aligned(q, 16) && is_aligned(k, 16) && is_aligned(v, 16);
+}
+// - and prompts that fill its chunks, by the average: the kernels for shorter chunks win with less, and a step that mixes a long prompt with
+// single tokens has a short average.  Time of those over time here, tiles (CTAs a sequence) T, on 148 SMs, prompts of one length:
+//     tokens          32    64    96   128   192   256   384   512   768
+//     state space, 128 states   16 x T 64   0.51  0.68  0.94  1.09  1.03  1.38  1.52  1.61  1.68      32 x T 64   0.43  0.58  0.83  0.99  0.96  1.28  1.43
+//     state space,  64 states   16 x T 64   0.39  0.49  0.64  0.79  0.72  0.94  1.03  1.09  1.14       8 x T 32   0.52  0.64  0.82  0.95  0.86  1.07  1.18
+//     matrix memory, 128        16 x T 48   0.53  0.73  0.93  1.12  1.06  1.34  1.43  1.48  1.57       4 x T 48   0.66  0.82  0.94  1.12  0.96  1.17  1.27
+//     matrix memory,  64         6 x T 32   0.68  0.73  0.84  0.95  0.84  0.96  1.00  1.00  1.02      32 x T  8   0.60  0.71  0.83  0.89  0.84  0.96  1.03
+//   every tile with an SM to itself: state space 0.86 / 1.07 / 1.43 at 32 / 64 / 96 tokens; matrix memory 0.83 / 0.91 / 1.00 and 0.93 to 1.39 at 160
+// One long prompt beside n - 1 single tokens, average 96: 0.64 to 0.74 (state space, which cuts the long one into segments), 1.5 to 2.0 (matrix
+// memory, whose old kernel does not); average 192 and up: faster here, or cut into segments (state_space.cu).
+static inline bool decay_chunks_filled(bool exp_gates, int n, int tokens, int num_seqs, int64_t tiles) {
+  const bool alone = num_seqs * tiles <= sm_count();
+  return tokens >= (alone && !exp_gates ? 64ll : alone || n == 128 ? 200ll : 512ll) * num_seqs;
 }
 
 template <int KB, bool EXP, bool STATES>

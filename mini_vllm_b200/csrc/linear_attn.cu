@@ -368,7 +368,8 @@ static int launch_linear(const LinearParams& p, cudaStream_t st) {
   if (p.heads > 65535 || p.num_seqs > 65535) return kUnsupportedShape;
   int rc = kUnsupportedShape;
   if constexpr (sizeof(T) == 2) {
-    if (EXP && decay_chunks_fit(p.q, p.k, p.v, p.qkv_stride, p.dim, p.vdim, p.tokens, p.num_seqs, p.heads)) {
+    if (EXP && decay_chunks_take(p.dim, p.vdim) && decay_chunks_read(p.q, p.k, p.v, p.qkv_stride) &&
+        decay_chunks_filled(true, p.dim, p.tokens, p.num_seqs, static_cast<int64_t>(p.heads) * (p.vdim / 64 + 1))) {
       rc = p.dim == 64 ? launch_mlstm_wide<1>(p, st) : launch_mlstm_wide<2>(p, st);
       return rc == kOk ? launch_linear_norm<T, EXP>(p, st) : rc;
     }

@@ -542,23 +542,30 @@ static int launch_ssd_step(const SsdParams& p, cudaStream_t st) {
 }
 
 // Segment length of a ragged step (0: whole sequences).  Worth its first pass, about half of the second's work, where the longest
-// sequence would be walked for twice as long as an even share of all tokens takes: two CTAs of 64 columns fit an SM.
-static int ssd_segment(int tokens, int longest, int heads, int vdim) {
-  const int64_t work = static_cast<int64_t>(tokens) * heads * ((vdim + 63) / 64), room = 2 * sm_count();
+// sequence would be walked for twice as long as an even share of all tokens takes.  tiles: CTAs of 64 columns a sequence; room: those that
+// run at once, two per SM here.
+static int ssd_even_segment(int tokens, int longest, int64_t tiles, int64_t room) {
+  const int64_t work = tokens * tiles;
   if (longest < 1024 || longest > tokens || longest * room <= 2 * work) return 0;
   int seg = 256;
   while (seg < 1024 && work / (2 * seg) >= 2 * room) seg *= 2;
   return seg;
 }
+static int ssd_segment(int tokens, int longest, int heads, int vdim) {
+  return ssd_even_segment(tokens, longest, static_cast<int64_t>(heads) * ((vdim + 63) / 64), 2 * sm_count());
+}
 static int64_t ssd_segment_slots(int tokens, int num_seqs, int seg) { return tokens / seg + num_seqs; }
 
-// The same for decay_chunk_kernel, which has an SM to itself
-static int ssd_wide_segment(int tokens, int longest, int heads, int vdim) {
-  const int64_t work = static_cast<int64_t>(tokens) * heads * (vdim / 64), room = sm_count();
-  if (longest < 1024 || longest > tokens || longest * room <= 2 * work) return 0;
-  int seg = 256;
-  while (seg < 1024 && work / (2 * seg) >= 2 * room) seg *= 2;
-  return seg;
+// Whether a step is one for decay_chunk_kernel, which has an SM to itself, and its segment length there.  A segment costs that kernel its set-up
+// once more, so segments are taken if all of them run at once or sequences are long on average, and with 128 states.  Time of ssd_chunk_kernel
+// (with its own segments) over time here, one long sequence beside n - 1 single tokens: 64 heads of 64, 128 states, n = 1 / 4 / 8: 1.15 / 1.24 /
+// 1.25 at 768 to 1,024 tokens on average, but 0.87 / 0.94 for n = 6 at 192 / 384; 8 heads, where all run at once: 1.7 to 1.9, else 0.86 to
+// 0.97 up to 512; 64 states: 0.61 to 1.05 throughout.
+static bool ssd_wide(int tokens, int num_seqs, int longest, int heads, int n, int vdim, int& seg) {
+  const int64_t tiles = static_cast<int64_t>(heads) * (vdim / 64);
+  if (!decay_chunks_take(n, vdim) || !decay_chunks_filled(false, n, tokens, num_seqs, tiles)) return false;
+  seg = ssd_even_segment(tokens, longest, tiles, sm_count());
+  return seg == 0 || (n == 128 && (ssd_segment_slots(tokens, num_seqs, seg) * tiles <= sm_count() || tokens >= 768ll * num_seqs));
 }
 
 template <int KS, int WARPS, bool STATES>
@@ -747,10 +754,12 @@ extern "C" size_t mvb_state_space_scratch_bytes(int dtype, int num_tokens, int n
                                                 int ragged) {
   using namespace mvb;
   if (!ragged || dtype != kBf16 || num_seqs <= 0 || heads <= 0 || num_states <= 0 || vdim <= 0) return 0;
-  // alignment, which decides between the kernels, is not known here: enough for either
+  // alignment, which also decides between the kernels, is not known here: enough for either
   int64_t slots = 0;
-  for (int seg : {ssd_segment(num_tokens, longest, heads, vdim), ssd_wide_segment(num_tokens, longest, heads, vdim)})
-    if (seg != 0) slots = std::max(slots, ssd_segment_slots(num_tokens, num_seqs, seg));
+  int seg = ssd_segment(num_tokens, longest, heads, vdim), wide_seg = 0;
+  if (seg != 0) slots = ssd_segment_slots(num_tokens, num_seqs, seg);
+  if (ssd_wide(num_tokens, num_seqs, longest, heads, num_states, vdim, wide_seg) && wide_seg != 0)
+    slots = std::max(slots, ssd_segment_slots(num_tokens, num_seqs, wide_seg));
   return static_cast<size_t>(slots) * heads * (static_cast<size_t>(num_states) * ((vdim + 3) / 4 * 4) + 1) * sizeof(float);
 }
 
@@ -773,9 +782,9 @@ extern "C" int mvb_state_space(int dtype, const void* x, const void* b, const vo
   SsdParams p{x, b, c, xbc_row_stride, dt, dt_row_stride, dt_bias, a_log2e, d, y, y_row_stride, state, state_slots, num_slots,
                     cu_seqlens_q, positions, num_seqs, num_tokens, heads, heads / groups, num_states, vdim, (vdim + 3) / 4 * 4, vec, 0, nullptr,
               nullptr, dev_status};
-  const bool wide = dtype == kBf16 && cu_seqlens_q != nullptr && vec && decay_chunks_fit(c, b, x, xbc_row_stride, num_states, vdim, num_tokens, num_seqs, heads);
-  if (dtype == kBf16 && cu_seqlens_q != nullptr)
-    p.seg = wide ? ssd_wide_segment(num_tokens, longest, heads, vdim) : ssd_segment(num_tokens, longest, heads, vdim);
+  const bool chunks = dtype == kBf16 && cu_seqlens_q != nullptr;
+  const bool wide = chunks && vec && decay_chunks_read(c, b, x, xbc_row_stride) && ssd_wide(num_tokens, num_seqs, longest, heads, num_states, vdim, p.seg);
+  if (chunks && !wide) p.seg = ssd_segment(num_tokens, longest, heads, vdim);
   if (p.seg != 0) {
     if (!scratch || scratch_bytes < mvb_state_space_scratch_bytes(dtype, num_tokens, num_seqs, longest, heads, num_states, vdim, 1)) return kInvalidArgument;
     if (!is_aligned(scratch, 16)) return kMisaligned;

@@ -58,7 +58,7 @@ def test_a_neighbour_full_of_infinities(cuda):
 @pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128), (128, 64), (64, 192)])
 @pytest.mark.parametrize("f_bias,swing", [(4.0, 1.0), (-8.0, 6.0), (0.0, 20.0)])
 def test_matrix_memory_edges(cuda, dim, vdim, f_bias, swing):
-    g, heads, cap, lens = gen(dim + vdim), 3, 15.0, [1, 31, 127, 128, 129, 300]
+    g, heads, cap, lens = gen(dim + vdim), 3, 15.0, [1, 31, 127, 128, 129, 300, 700, 256]
     mk = lambda *s: torch.randn(*s, generator=g).to(BF)
     seqs = [{"q": mk(t, heads, dim), "k": mk(t, heads, dim), "v": mk(t, heads, vdim), "gate": mk(t, heads * vdim),
              "f": (mk(t, heads) * swing).to(BF), "i": (mk(t, heads) * swing).to(BF)} for t in lens]
@@ -130,14 +130,14 @@ def memory_step(cuda, lens, heads, dim, vdim, f_bias, i_bias, eps, states=None, 
 def test_matrix_memory_goes_on(cuda, dim, vdim):
     """Prompts behind a state of random values, whose normaliser comes from memory while the first products already run: outputs (an eps that
     keeps their size visible), memory, normaliser and maximum against the oracle."""
-    heads, lens, slots, g = 16, [130, 5, 128, 257, 64, 200], [3, 6, 0, 1, 7, 4], gen(3)
+    heads, lens, slots, g = 8, [330, 5, 128, 257, 364, 200], [3, 6, 0, 1, 7, 4], gen(3)
     states = tuple(x.to(cuda) for x in (torch.randn(9, heads, dim, vdim, generator=g), torch.randn(9, heads, dim, generator=g), torch.randn(9, heads, generator=g)))
     torch.empty(64 << 20, device=cuda).zero_()                       # the states are no longer in a cache
     got, want, behind, status = memory_step(cuda, lens, heads, dim, vdim, 4.0, -1.0, 0.5, states, slots, [7, 9, 0, 3, 1, 2])
     ops.check_status(status)
     for j, slot in enumerate(slots):
         assert rel(got[j], want[j]) < 8e-3
-        # factors of 16 bits, fp32 sums of up to 257 terms
+        # factors of 16 bits, fp32 sums of up to 364 terms
         assert all(rel(states[m][slot], behind[j][m]) < 3e-5 for m in range(3))
 
 
@@ -151,11 +151,11 @@ def test_a_normaliser_that_all_but_cancels(cuda, dim, vdim):
         s["k"][:] = 0
         s["k"][40], s["k"][41] = k * 1000, -k * 1000         # (n . q stays above the floor of its size)
         s["q"] *= 1000
-    got, want, _, status = memory_step(cuda, [100, 128], 16, dim, vdim, 11.9, 0.0, 1e12, edit=edit)
+    got, want, _, status = memory_step(cuda, [200, 230], 16, dim, vdim, 11.9, 0.0, 1e12, edit=edit)
     ops.check_status(status)
     errs = []
     for x, y in zip(got, want):
-        x, y = (z.view(-1, 16, vdim)[41:] for z in (x, y))
+        x, y = (z.view(-1, 16, vdim)[41:128] for z in (x, y))
         errs.append((x * y).sum(-1) / (y * y).sum(-1) - 1)             # of the size of a head's row: the rounding to bf16 averages out
     err = float(torch.cat(errs).pow(2).mean().sqrt())
     assert err < 1e-2, err
@@ -211,16 +211,16 @@ def test_weak_decays_behind_strong_ones(cuda, n, vdim):
     y, S = space_walk(seqs[0], 0.0, a)
     assert off(got[0], y) < 4e-3
     err = off(state[0], S)
-    assert err < 2 ** -18, err
+    assert err < 2 ** -17, err
 
 
 @pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128)])
 def test_weak_forget_gates_behind_strong_ones(cuda, dim, vdim):
     """The same of the matrix memory; its gates' functions are those of CUDA, exact to a few ulps."""
     def edit(s):
-        s["f"][:96], s["f"][96:128], s["i"] = -40, 8, s["i"] * 0.1
+        s["f"][:224], s["f"][224:256], s["i"] = -40, 8, s["i"] * 0.1
     states = tuple(torch.zeros(*s, device=cuda) for s in ((1, 3, dim, vdim), (1, 3, dim), (1, 3)))
-    got, want, behind, status = memory_step(cuda, [128], 3, dim, vdim, 0.0, 0.0, 0.5, states, [0], edit=edit)
+    got, want, behind, status = memory_step(cuda, [256], 3, dim, vdim, 0.0, 0.0, 0.5, states, [0], edit=edit)
     ops.check_status(status)
     assert off(got[0], want[0]) < 4e-3
     errs = [off(x[0], y) for x, y in zip(states, behind[0])]

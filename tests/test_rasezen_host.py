@@ -213,3 +213,13 @@ def test_mistakes_show_in_the_logits(name):
     toks = [(7 * i * i + 3 * i) % 96 for i in range(80)]
     want = plain.OracleRasezen(w, cfg).forward(toks)
     assert row_errors(plain.OracleRasezen(ww, wrong).forward(toks), want).max() > 3e-3
+
+
+def test_segments_are_asked_for_where_they_are_walked():
+    """Scratch of a state-space step: none where no kernel would cut its sequences, and enough where one does."""
+    from mini_vllm_b200 import _cabi
+    need = _cabi.load().mvb_state_space_scratch_bytes
+    assert need(0, 1100, 2, 1050, 256, 128, 32, 1) == 0               # SMs enough have work, and 32 columns are no tile of the wide kernel
+    assert need(0, 1100, 2, 1050, 256, 96, 64, 1) == 0                # nor 96 states
+    assert need(0, 4096, 1, 4096, 8, 128, 64, 1) >= (4096 // 256 + 1) * 8 * (128 * 64 + 1) * 4
+    assert need(0, 4096, 1, 4096, 8, 128, 64, 0) == 0 and need(1, 4096, 1, 4096, 8, 128, 64, 1) == 0
