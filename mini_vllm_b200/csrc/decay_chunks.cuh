@@ -26,10 +26,10 @@
 //   warp 16       TMA: q, k and v of the next chunk while this one is worked on (two stages; one of q where the third part takes its place)
 //   warps 17, 19  tcgen05.mma
 //   warp 18       gates of the next chunk
-// What bounds it: 2,048 tensor-core cycles per 128 tokens, head and 64 columns (N = 128), about 3,200 with their operands' way through
-// shared memory, and 3,000 issue slots of the warps around them, which also wait for one another.  mma.sync, which this replaces for prompts
-// that fill its chunks, took its own issue for four fifths of the time.  Measured: 6 prompts of 500 to 2,500 tokens (10,148 in all), state space
-// with 64 heads of 64 x 128: 153 us (280 before); matrix memory with 16 heads of 128 x 128 and its norm: 220 us (387 before).
+// What bounds it: the issue of the warps that make M and the scaled values; by operations the products need 2,048 tensor-core cycles per 128
+// tokens, head and 64 columns.  mma.sync, which this replaces for prompts that fill its chunks, took its own issue for most of the time.
+// Measured: 6 prompts of 500 to 2,500 tokens (10,148 in all), state space with 64 heads of 64 x 128: 158 us (280 before); matrix memory with 16
+// heads of 128 x 128 and its norm: 242 us (387 before).
 #pragma once
 #include "chunk_common.cuh"
 #include "host_util.cuh"
@@ -393,8 +393,7 @@ decay_chunk_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     if (STATES && blockIdx.x == 0 && lane == 0) p.seg_keep[static_cast<int64_t>(blockIdx.z) * p.heads + h] = fast_exp2(kept);
   } else if (warp < 8) {
     // ============================ M, scaled values ======================================================
-    // Loops instead of straight code wherever registers allow it: with everything unrolled the warps of this kernel waited for
-    // instructions five times as long as they issued.
+    // Loops instead of straight code wherever registers allow it: with everything unrolled the state space's case took 236 us instead of 153.
     const int quad = warp & 3, row = quad * 32 + lane, half = warp >> 2, sw = (row & 7) << 4;
     auto r_of = [&](const float* tab, int t) { return EXP ? tab[C::X3 + t] : -tab[C::E + t]; };
     auto scale_values = [&](int c) {

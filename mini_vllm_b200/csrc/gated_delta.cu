@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const DeltaParams p, in
 }
 
 // The same for many sequences: one CTA per SM walks (sequence, head) pairs while bulk copies bring the states of the next two and take the
-// last one's back, so that HBM waits less for arithmetic.  The sums run in the order of delta_step_kernel.
+// last one's back, so that HBM waits less for arithmetic.  The sums run in the order of delta_step_kernel where that has 16 rows a thread.
 //   warps 0..7   arithmetic: thread = 16 rows x 4 columns     warp 8   copies
 // 256 sequences x 16 heads of 128 x 128: 112 us (delta_step_kernel 124; HBM's floor 83).  With 512 threads 126, with two groups of 256 on
 // alternate pairs, which leaves one stage to load ahead, 147: the three stages' round trip of copies bounds it.
