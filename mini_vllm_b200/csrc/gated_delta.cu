@@ -52,16 +52,19 @@ __device__ __forceinline__ int64_t delta_slot(const DeltaParams& p, int s) {
 __device__ __forceinline__ float decay_of(float raw, float bias, float exp_a) { return expf(-exp_a * softplus_f(raw + bias)); }
 
 // ---- one token per sequence ------------------------------------------------------------------------------
+// floats in front of the partial sums, which are read and written four at a time: q, k and g rounded up (dim need not be a multiple of four)
+__host__ __device__ inline int step_red_at(int dim) { return (3 * dim + 3) / 4 * 4; }
+
 template <class T, int RPT>
 __global__ void __launch_bounds__(512) delta_step_kernel(const DeltaParams p, int tile_cols) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int s = blockIdx.z, h = blockIdx.x, kvh = h / (p.heads / p.kv_heads);
   const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   const int col0 = blockIdx.y * tile_cols, cols = min(tile_cols, p.vp - col0), quads = tile_cols / 4;
   float* q_s = sm;                              // [dim]
   float* k_s = q_s + p.dim;
   float* g_s = k_s + p.dim;
-  float* red = g_s + p.dim;                     // [row groups][tile_cols]
+  float* red = sm + step_red_at(p.dim);         // [row groups][tile_cols]
   __shared__ float wsum[2][16];
   const int64_t slot = delta_slot(p, s);
   const bool fresh = slot < 0 || p.positions[s] == 0;
@@ -495,7 +498,7 @@ static int launch_step(const DeltaParams& p, cudaStream_t st) {
     const int row_groups = (p.dim + RPT - 1) / RPT;
     int nt = (row_groups * quads + 31) / 32 * 32;
     if (nt < (tile + 31) / 32 * 32) nt = (tile + 31) / 32 * 32;  // a thread per column at the end
-    const size_t smem = (3 * static_cast<size_t>(p.dim) + static_cast<size_t>(row_groups) * tile) * sizeof(float);
+    const size_t smem = (static_cast<size_t>(step_red_at(p.dim)) + static_cast<size_t>(row_groups) * tile) * sizeof(float);
     if (nt > 512 || smem > 47 * 1024) return kUnsupportedShape;
     delta_step_kernel<T, RPT><<<dim3(p.heads, tiles, p.num_seqs), nt, smem, st>>>(p, tile);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;

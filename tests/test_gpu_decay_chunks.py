@@ -216,11 +216,11 @@ def test_weak_decays_behind_strong_ones(cuda, n, vdim):
 
 @pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128)])
 def test_weak_forget_gates_behind_strong_ones(cuda, dim, vdim):
-    """The same of the matrix memory; its gates' functions are those of CUDA, exact to a few ulps."""
+    """The same of the matrix memory (the first of two prompts); its gates' functions are those of CUDA, exact to a few ulps."""
     def edit(s):
-        s["f"][:224], s["f"][224:256], s["i"] = -40, 8, s["i"] * 0.1
-    states = tuple(torch.zeros(*s, device=cuda) for s in ((1, 3, dim, vdim), (1, 3, dim), (1, 3)))
-    got, want, behind, status = memory_step(cuda, [256], 3, dim, vdim, 0.0, 0.0, 0.5, states, [0], edit=edit)
+        s["f"][:96], s["f"][96:128], s["i"] = -40, 8, s["i"] * 0.1
+    states = tuple(torch.zeros(*s, device=cuda) for s in ((2, 3, dim, vdim), (2, 3, dim), (2, 3)))
+    got, want, behind, status = memory_step(cuda, [128, 300], 3, dim, vdim, 0.0, 0.0, 0.5, states, [0, 1], edit=edit)
     ops.check_status(status)
     assert off(got[0], want[0]) < 4e-3
     errs = [off(x[0], y) for x, y in zip(states, behind[0])]
